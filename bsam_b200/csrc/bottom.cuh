@@ -2,20 +2,20 @@
 //
 // Below a few thousand cells a level is far too small to fill the GPU, and a
 // launch per colour pass and per transfer makes the coarse levels of a
-// V-cycle launch-latency bound.  k_bottom runs AFASVcycle (afas:488-521) for
-// a whole chain of small uniform levels -- from the chain's top patch down to
-// the coarsest level and back -- inside one CTA, with __syncthreads between
-// the phases the reference separates (every colour pass, restriction, coarse
-// load, correction).  The per-cell arithmetic is the same device code as the
-// grid kernels, so the results are identical.  One CTA per chain: a batch of
-// independent problems runs its bottoms side by side in one launch.
+// V-cycle launch-latency bound.  The batch's kb_bottom (batch.cuh) runs
+// AFASVcycle (afas:488-521) for a whole chain of small uniform levels -- from
+// the chain's top patch down to the coarsest level and back -- inside one CTA,
+// with __syncthreads between the phases the reference separates (every colour
+// pass, restriction, coarse load, correction).  The per-cell arithmetic is the
+// same device code as the grid kernels, so the results are identical.  One CTA
+// per chain: a batch of independent problems runs its bottoms side by side in
+// one launch.
 #pragma once
 #include "kernels.cuh"
 
 namespace bsam {
 
-constexpr int BOTTOM_THREADS = 512;
-constexpr int BOTTOM_MAX_CELLS = 4096;  // largest level handled by k_bottom
+constexpr int BOTTOM_MAX_CELLS = 4096;  // largest level of a bottom chain
 constexpr int BOTTOM_MAX_DEPTH = 16;
 
 template <class T, int D>
@@ -96,19 +96,6 @@ __device__ __forceinline__ void bottom_chain(const DevPatch* __restrict__ PT, in
     block_correct<T, D>(P, Q);
     block_relax<T, D>(P, nu);
   }
-}
-
-// tops[b]: the top patch of chain b; the chain follows parent links down to
-// the coarsest level.  nu = nsmoothingpasses.  Chains whose top is inactive
-// (finished batch slots) are skipped.
-template <class T, int D>
-__global__ void __launch_bounds__(BOTTOM_THREADS)
-    k_bottom(const DevPatch* __restrict__ PT, const int* __restrict__ tops, int nu) {
-  __shared__ int chain[BOTTOM_MAX_DEPTH];
-  __shared__ int depth;
-  const int top = tops[blockIdx.x];
-  if (!PT[top].active) return;
-  bottom_chain<T, D>(PT, top, nu, chain, depth);
 }
 
 }  // namespace bsam

@@ -23,6 +23,8 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -30,7 +32,7 @@
 #include "bsam_types.h"
 #include "kernels.cuh"
 #include "smooth_fused.cuh"
-#include "bottom.cuh"
+#include "chain.cuh"
 #include "mixed.cuh"
 #include "amr.cuh"
 #include "regrid.cuh"
@@ -43,9 +45,10 @@ namespace {
 
 // Levels with at most this many cells per patch stay FP64 in the mixed form.
 constexpr int64_t MIXED_FP64_CELLS = 4096;
-// Default largest level of the one-CTA bottom chain, per dimensionality.
-constexpr int DEFAULT_BOTTOM_CELLS_2D = 1024;
-constexpr int DEFAULT_BOTTOM_CELLS_3D = 512;
+// Largest level of the bottom chain where the caller asks for fused stages
+// (levels above it may run them), per dimensionality.
+constexpr int FUSED_BOTTOM_CELLS_2D = 1024;
+constexpr int FUSED_BOTTOM_CELLS_3D = 512;
 
 struct LevelPlan {
   int level = 0;
@@ -153,9 +156,12 @@ struct bsam_gpu {
   // Fused stages off by default: at L2-resident sizes the per-pass kernels
   // are faster; tests and tuning switch them on.
   bsam_tuning tuning{0, 64, 0, 0, 0, {0, 0, 0}};
-  int bottom_level = -1000;  // levels <= this run inside k_bottom
-  int* d_tops = nullptr;     // top patch of each k_bottom chain
-  int ntops = 0;
+  int bottom_level = -1000;  // levels <= this run inside k_chain
+  ChainPlan* d_chains = nullptr;  // one plan per patch of that level
+  int nchains = 0, chain_ctas = 1;
+  size_t chain_smem = 0;
+  bool chain_loop = false;   // the chain is the whole solve: V-cycle loop in the kernel
+  int max_cluster = 1;       // CTAs of the largest cluster the device runs
   double denom = 1.0;        // nrvars * cells of the finest level (ErrorAFAS)
   cudaGraphExec_t step_exec = nullptr;  // V-cycle loop graph (built lazily)
   int graph_kernels_per_vcycle = 0;
@@ -403,18 +409,31 @@ void transfer(bsam_gpu* h, int level, int what) {
   }
 }
 
+// The chains below and including bottom_level (chain.cuh): one V-cycle, or
+// with loop.maxv > 0 MultigridIterations' whole loop.
+void launch_chain(bsam_gpu* h, const ChainLoop& loop) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)(h->nchains * h->chain_ctas));
+  cfg.blockDim = dim3(CHAIN_THREADS);
+  cfg.dynamicSmemBytes = h->chain_smem;
+  cfg.stream = h->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = (unsigned)h->chain_ctas;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  auto k = h->rp.ndims == 2 ? (h->mixed ? k_chain<2, true> : k_chain<2, false>)
+                            : (h->mixed ? k_chain<3, true> : k_chain<3, false>);
+  (void)cudaLaunchKernelEx(&cfg, k, (const DevPatch*)h->d_patches,
+                           (const ChainPlan*)h->d_chains, loop);
+  ++h->stats.launches;
+}
+
 // AFASVcycle (afas:488-521).
 void vcycle(bsam_gpu* h, int level) {
   if (level == h->bottom_level) {
-    // AFASVcycle(level) down to the coarsest level in one launch (bottom.cuh);
-    // bottom levels are FP64 in both forms.
-    if (h->rp.ndims == 2)
-      k_bottom<double, 2><<<h->ntops, BOTTOM_THREADS, 0, h->stream>>>(h->d_patches, h->d_tops,
-                                                                      h->rp.nsmoothingpasses);
-    else
-      k_bottom<double, 3><<<h->ntops, BOTTOM_THREADS, 0, h->stream>>>(h->d_patches, h->d_tops,
-                                                                      h->rp.nsmoothingpasses);
-    ++h->stats.launches;
+    launch_chain(h, ChainLoop{});  // AFASVcycle(level) down to the coarsest level
     return;
   }
   relax_level(h, level, 0);  // LevelRelax (afas:499)
@@ -705,7 +724,7 @@ int bsam_gpu_create(bsam_gpu** out, int device, const bsam_run_params* p) {
 }
 
 static void free_hierarchy(bsam_gpu* h) {
-  // d_items, d_tmaps, d_tops, d_patches, d_partials, d_qold_spans, d_plist
+  // d_items, d_tmaps, d_chains, d_patches, d_partials, d_qold_spans, d_plist
   // and d_ovl point into d_meta, which the handle keeps.
   h->d_tmaps = nullptr;
   if (h->step_exec) cudaGraphExecDestroy(h->step_exec);
@@ -714,8 +733,8 @@ static void free_hierarchy(bsam_gpu* h) {
   h->nqold_spans = 0;
   h->qold_span_max = 0;
   h->d_items = nullptr;
-  h->d_tops = nullptr;
-  h->ntops = 0;
+  h->d_chains = nullptr;
+  h->nchains = 0;
   h->step_exec = nullptr;
   h->d_arena = nullptr;
   h->d_patches = nullptr;
@@ -733,6 +752,90 @@ static void free_hierarchy(bsam_gpu* h) {
   h->desc.clear();
   h->field_elems.clear();
   h->have_hierarchy = false;
+}
+
+// Sets k_chain's attributes and returns the CTAs of the largest cluster of it
+// that the device can hold (16 need a GPC with 16 free SMs, 8 always fit;
+// negative: a CUDA error).  The attributes belong to the device's context and
+// the answer to the device, so both are settled once per device: the queries
+// take milliseconds.
+static int chain_cluster(int device) {
+  static std::mutex mutex;
+  static std::map<int, int> known;
+  std::lock_guard<std::mutex> lock(mutex);
+  const auto it = known.find(device);
+  if (it != known.end()) return it->second;
+  int most = CHAIN_MAX_CTAS;
+  auto one = [&](auto k) {
+    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)CHAIN_SMEM_MAX) != cudaSuccess ||
+        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+      return false;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(CHAIN_MAX_CTAS);
+    cfg.blockDim = dim3(CHAIN_THREADS);
+    cfg.dynamicSmemBytes = CHAIN_SMEM_MAX;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = CHAIN_MAX_CTAS;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      most = 8;
+    }
+    return true;
+  };
+  if (!one(k_chain<2, false>) || !one(k_chain<2, true>) || !one(k_chain<3, false>) ||
+      !one(k_chain<3, true>))
+    return -1;
+  known[device] = most;
+  return most;
+}
+
+// The chains whose tops are the patches of `level`, each following parent
+// links to the coarsest level, laid out in shared memory.  False when one
+// does not fit, when a top exceeds bmax cells, or when two chains meet.
+static bool find_chains(bsam_gpu* h, int npatch, const bsam_patch_desc* patches, int level,
+                        int64_t bmax, int64_t fp64_cells, bool loop,
+                        std::vector<std::vector<int>>& chains, std::vector<ChainPlan>& plans) {
+  const int nd = h->rp.ndims;
+  chains.clear();
+  plans.clear();
+  std::vector<char> seen(npatch, 0);
+  for (int p = 0; p < npatch; ++p) {
+    if (patches[p].level != level) continue;
+    std::vector<int> chain, prec;
+    std::vector<std::array<int, 3>> n;
+    for (int r = p; r >= 0; r = patches[r].parent) {
+      if (r >= npatch || seen[r] || (int)chain.size() == CHAIN_MAX_LEVELS) {
+        chains.clear();
+        plans.clear();
+        return false;
+      }
+      seen[r] = 1;
+      chain.push_back(r);
+      std::array<int, 3> e{1, 1, 1};
+      for (int d = 0; d < nd; ++d) e[d] = patches[r].mx[d];
+      const int64_t cells = (int64_t)e[0] * e[1] * e[2];
+      n.push_back(e);
+      prec.push_back(!h->mixed || cells <= fp64_cells ? PREC_F64 : PREC_F32);
+    }
+    ChainPlan C;
+    bool ok = cells_of(n[0].data(), nd) <= bmax;
+    for (auto& e : n) ok = ok && e[0] > 0 && e[1] > 0 && e[2] > 0;
+    if (!ok || !chain_layout(nd, n, prec, h->mixed, h->rp.nsmoothingpasses, h->max_cluster, loop,
+                             C)) {
+      chains.clear();
+      plans.clear();
+      return false;
+    }
+    chains.push_back(chain);
+    plans.push_back(C);
+  }
+  return !plans.empty();
 }
 
 int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patches,
@@ -755,34 +858,33 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
   for (int l = minlevel; l <= finestlevel; ++l) plan(h, l).level = l;
   h->desc.assign(patches, patches + npatch);
 
-  // Bottom level: the finest level such that it and every coarser level hold
-  // at most bottom_cells cells per patch (uniform hierarchies only).
-  h->bottom_level = -1000;
-  // Default: chains from 1024 cells (2D) or 512 (3D) down.  The one-CTA
-  // chain runs on a single SM, so a larger top level there (4096 cells: 64^2,
-  // 16^3) leaves the rest of the GPU idle for longer than the grid kernels
-  // take for it (measured: 128^2 FP64 829 -> 915 time-steps/s; 16^3 .. 1^3
-  // alone was a quarter of a 128^3 V-cycle).
+  // Mixed form: levels at or below this size stay FP64: 4096 cells, or the
+  // size the caller gives for the bottom chain.
   const bool dflt = h->tuning.bottom_cells == 0;
-  const int bmax = dflt ? (nd == 3 ? DEFAULT_BOTTOM_CELLS_3D : DEFAULT_BOTTOM_CELLS_2D)
-                        : h->tuning.bottom_cells;
-  if (bmax > 0) {
-    // Only the root and the levels below it (one uniform patch each).
-    for (int l = minlevel; l <= std::min(finestlevel, 0); ++l) {
-      bool small = true;
-      for (int p = 0; p < npatch; ++p)
-        if (patches[p].level == l) small = small && cells_of(patches[p].mx, nd) <= bmax;
-      if (!small) break;
+  const int64_t fp64_cells = h->tuning.bottom_cells > 0 ? h->tuning.bottom_cells
+                                                        : MIXED_FP64_CELLS;
+  // Bottom level: the finest level from which every chain of levels down to
+  // the coarsest fits in the shared memory of one cluster (chain.cuh).  A
+  // pass costs less there than a launch per pass at every size that fits
+  // (128^2 FP64: 0.5 against 5.3 us; 32^3: 1.0 against 6.0 us), so the
+  // largest that fits is taken, within the caller's bottom_cells if given.
+  int64_t bmax = dflt ? INT64_MAX : h->tuning.bottom_cells;
+  if (dflt && h->tuning.fuse_smoother != 0)
+    bmax = nd == 3 ? FUSED_BOTTOM_CELLS_3D : FUSED_BOTTOM_CELLS_2D;
+  if ((h->max_cluster = chain_cluster(h->device)) < 0)
+    return fail(h, BSAM_ERR_CUDA, "the chain kernel's attributes were rejected");
+  h->bottom_level = -1000;
+  h->chain_loop = false;
+  std::vector<std::vector<int>> chains;  // per chain its patches, top first
+  std::vector<ChainPlan> plans;
+  for (int l = std::min(finestlevel, 0); bmax > 0 && l >= minlevel; --l) {
+    const bool loop = l == finestlevel && !h->mixed && finestlevel == 0;
+    if (find_chains(h, npatch, patches, l, bmax, fp64_cells, loop, chains, plans)) {
       h->bottom_level = l;
+      h->chain_loop = loop && chains.size() == 1;
+      break;
     }
-    if (h->bottom_level - minlevel + 1 > BOTTOM_MAX_DEPTH) h->bottom_level = -1000;
   }
-  // Mixed form: levels at or below this size stay FP64 -- the levels the
-  // bottom kernel runs, including the coarsest; 4096 cells under the default
-  // bottom size and when the bottom kernel is switched off (the levels
-  // between the default bottom and 4096 cells run FP64 grid kernels, which
-  // give the bottom kernel's bits).
-  const int64_t fp64_cells = (!dflt && bmax > 0) ? (int64_t)bmax : MIXED_FP64_CELLS;
 
   // Records: the caller's patches, then one twin per finest-level patch in
   // the mixed form.
@@ -1180,13 +1282,23 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     for (int p : h->masters) ncells += cells_of(h->hp[p].n, nd);
     h->denom = (double)(h->rp.nrvars * ncells);  // L2Error's integralresult(2)
   }
-  std::vector<int> tops;
-  if (h->bottom_level >= minlevel) {
-    tops = plan(h, h->bottom_level).patches;
-    for (int p : tops)
-      if (h->hp[p].prec != PREC_F64) return fail(h, BSAM_ERR_ARG, "bottom levels must be FP64");
-    h->ntops = (int)tops.size();
+  h->nchains = (int)plans.size();
+  h->chain_ctas = 1;
+  h->chain_smem = 0;
+  for (size_t c = 0; c < plans.size(); ++c) {
+    ChainPlan& C = plans[c];
+    h->chain_ctas = std::max(h->chain_ctas, C.ctas);
+    h->chain_smem = std::max(h->chain_smem, (size_t)C.smem);
+    for (int l = 0; l < C.nlev; ++l) {
+      const int p = chains[c][l];
+      const int r = twin_of[p] >= 0 ? twin_of[p] : p;
+      const DevPatch& P = h->hp[r];
+      if (P.prec != C.L[l].prec || P.delta != C.L[l].delta)
+        return fail(h, BSAM_ERR_ARG, "a chain level's form differs from its record's");
+      chain_faces(C, l, r, P);
+    }
   }
+  for (ChainPlan& C : plans) C.ctas = h->chain_ctas;
   // The tables' layout in d_meta (256-byte aligned pieces), the buffer grown
   // when too small, then the pointers, and one copy of the host image.
   {
@@ -1204,7 +1316,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     const size_t o_ovl_rng = place(sizeof(int2) * ovl_range.size());
     const size_t o_qold = place(sizeof(CopySpan) * qold_spans.size());
     const size_t o_maps = place(sizeof(CUtensorMap) * maps.size());
-    const size_t o_tops = place(sizeof(int) * tops.size());
+    const size_t o_chains = place(sizeof(ChainPlan) * plans.size());
     const size_t o_part = place(sizeof(double) * h->max_items);
     const size_t total_meta = off;
     if (total_meta > h->meta_cap) {
@@ -1222,7 +1334,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     h->d_ovl = ovl_all.empty() ? nullptr : reinterpret_cast<OverlapCopy*>(base + o_ovl);
     h->d_qold_spans = qold_spans.empty() ? nullptr : reinterpret_cast<CopySpan*>(base + o_qold);
     h->d_tmaps = maps.empty() ? nullptr : reinterpret_cast<CUtensorMap*>(base + o_maps);
-    h->d_tops = tops.empty() ? nullptr : reinterpret_cast<int*>(base + o_tops);
+    h->d_chains = plans.empty() ? nullptr : reinterpret_cast<ChainPlan*>(base + o_chains);
     h->d_partials = reinterpret_cast<double*>(base + o_part);
     h->d_patches = reinterpret_cast<DevPatch*>(base + o_patches);
     for (size_t k = 0; k < fused_recs.size(); ++k) h->hp[fused_recs[k]].tmaps = h->d_tmaps + 7 * k;
@@ -1256,7 +1368,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     put(o_ovl_rng, ovl_range.data(), sizeof(int2) * ovl_range.size());
     put(o_qold, qold_spans.data(), sizeof(CopySpan) * qold_spans.size());
     put(o_maps, maps.data(), sizeof(CUtensorMap) * maps.size());
-    put(o_tops, tops.data(), sizeof(int) * tops.size());
+    put(o_chains, plans.data(), sizeof(ChainPlan) * plans.size());
     const int urc = h2d_bounce(h, h->d_meta, img.data(), img.size());
     if (urc) return urc;
   }
@@ -1420,21 +1532,30 @@ int bsam_gpu_multigrid_iterations(bsam_gpu* h, int* nvcycles, double* residual, 
   int it = 0, conv = 0;
   double res = 0.0;
   if (h->tuning.graph == 0 && !h->profiling) {
-    // The whole V-cycle loop as one graph launch (device-side WHILE node).
-    if (!h->step_exec) {
-      const int rc = build_step_graph(h);
-      if (rc) return rc;
+    if (h->chain_loop) {
+      // Every level in one cluster's shared memory: the loop is one launch.
+      launch_chain(h, ChainLoop{h->rp.maxvcycles, 0, h->rp.qerrortol, h->denom, h->d_status,
+                                h->d_trace});
+      CU(cudaGetLastError());
+      h->graph_kernels_per_vcycle = 0;
+    } else {
+      // The whole V-cycle loop as one graph launch (device-side WHILE node).
+      if (!h->step_exec) {
+        const int rc = build_step_graph(h);
+        if (rc) return rc;
+      }
+      k_mg_begin<<<1, 1, 0, h->stream>>>(h->d_status);
+      CU(cudaGetLastError());
+      CU(cudaGraphLaunch(h->step_exec, h->stream));
+      ++h->stats.launches;
     }
-    k_mg_begin<<<1, 1, 0, h->stream>>>(h->d_status);
-    CU(cudaGetLastError());
-    CU(cudaGraphLaunch(h->step_exec, h->stream));
     CU(cudaMemcpyAsync(h->h_status, h->d_status, sizeof(DevStatus), cudaMemcpyDeviceToHost,
                        h->stream));
     CU(cudaMemcpyAsync(h->h_trace, h->d_trace, sizeof(double) * h->rp.maxvcycles,
                        cudaMemcpyDeviceToHost, h->stream));
     CU(cudaStreamSynchronize(h->stream));
     it = std::max(1, std::min(h->h_status->iters, h->rp.maxvcycles));
-    h->stats.launches += 1 + (int64_t)h->graph_kernels_per_vcycle * h->h_status->iters;
+    h->stats.launches += (int64_t)h->graph_kernels_per_vcycle * h->h_status->iters;
     res = h->h_status->residual;
     h->trace.assign(h->h_trace, h->h_trace + it);
     if (nvcycles) *nvcycles = it;

@@ -81,11 +81,12 @@ int bsam_gpu_create(bsam_gpu** h, int device, const bsam_run_params* p);
  *   fuse_min_n     smallest extent per dimension of a fused level
  *   chunk          planes (3D) / rows (2D) per streaming chunk, 0 = automatic
  *   bottom_cells   levels of at most this many cells run their whole part of
- *                  the V-cycle in one single-CTA launch (at most 4096);
- *                  0 = default (1024 in 2D, 512 in 3D), -1 = never.  In the
- *                  mixed form these levels are FP64; under the default and
- *                  with -1, levels of at most 4096 cells are FP64 (the bits
- *                  do not depend on which of them run in the bottom launch)
+ *                  the V-cycle in one launch (a thread-block cluster, the
+ *                  levels in its shared memory) as far as they fit there;
+ *                  0 = default (as many levels as fit), -1 = never.  In the
+ *                  mixed form levels of at most bottom_cells are FP64; under
+ *                  the default and with -1, levels of at most 4096 cells are
+ *                  (the bits do not depend on which of them run in that launch)
  *   graph          0 = run the V-cycle loop of MultigridIterations as one
  *                  captured CUDA graph with a device-side WHILE node (one
  *                  launch per call); -1 = host loop (one launch per kernel,
