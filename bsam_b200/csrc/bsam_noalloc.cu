@@ -17,6 +17,7 @@
 // give wrong results; order such calls on one stream.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <mutex>
 
 #include "../../include/bsam_gpu.h"
@@ -27,8 +28,8 @@ using namespace bsam;
 
 namespace {
 
-// One partial sum per CTA (tile of 64 x 4 x 1 cells) plus the ticket of the
-// last-block-done reduction in the trailing 256 bytes.
+// Partial sums, one per CTA (at most one per tile of 64 x 4 x 1 cells), plus the
+// ticket of the last-block-done reduction in the trailing 256 bytes.
 constexpr int NOALLOC_MAX_TILES = BSAM_NOALLOC_MAX_TILES;
 constexpr int NOALLOC_TAIL_DOUBLES = 32;
 constexpr size_t NOALLOC_SCRATCH_BYTES =
@@ -60,39 +61,70 @@ int scratch_for_device(int device, double** out) {
   return BSAM_OK;
 }
 
-// Variant of k_resid_norm that reads the caller's Fortran-layout arrays and
-// reduces through the static scratch.  The tile of a CTA is derived from
-// blockIdx in the same x-fastest order as the library's work lists, so the
-// partial sums are combined in the same order as bsam_gpu_multigrid_iterations.
+// ErrorAFAS's norm over the caller's Fortran-layout arrays, reduced through the
+// static scratch.  A warp takes 32 columns and marches down `rows` rows, so that
+// a row of q is loaded once as the next row's centre and reused as south
+// neighbour; three CTAs per SM stay for the whole patch and take such pieces in
+// turn.  Bound by HBM latency: eight rows unrolled put the loads of eight rows
+// in flight, which pays more than warps (4096^2, 537 MB: 106 us = 5.1 TB/s with
+// eight rows and three CTAs; 126 with four rows and four CTAs, 156 with two and
+// eight; a CTA per 64 x 4 tile with its own reduction and ticket took 210).
+constexpr int NORM_WARPS = 8;
+constexpr int NORM_CTAS_PER_SM = 3;
 template <int D>
-__global__ void __launch_bounds__(BLOCK_THREADS)
+__global__ void __launch_bounds__(32 * NORM_WARPS, NORM_CTAS_PER_SM)
     k_resid_norm_noalloc(DevPatch P, const double* __restrict__ fbase, int64_t fsy,
-                         int64_t fsz, int64_t fcomp, int tiles_x, int tiles_y,
-                         double* __restrict__ scratch, double denom, double* __restrict__ out) {
-  const int b = blockIdx.x;
-  const int tx = b % tiles_x, ty = (b / tiles_x) % tiles_y, tz = b / (tiles_x * tiles_y);
-  const int j = ty * TILE_Y + threadIdx.y + 1;
-  const int k = (D == 3) ? tz + 1 : 0;
-  const int i0 = (tx * 32 + threadIdx.x) * 2 + 1;
-  const double* q0 = static_cast<const double*>(P.q[0]);
-  const double* q1 = static_cast<const double*>(P.q[1]);
+                         int64_t fsz, int64_t fcomp, int nseg, int nchunk, int rows,
+                         int64_t pieces, double* __restrict__ scratch, double denom, double* __restrict__ out) {
+  const int lane = threadIdx.x & 31;
   double acc = 0.0;
-  if (j <= P.n[1]) {
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      const int i = i0 + t;
-      if (i <= P.n[0]) {
-        Problem::Stencil<double, D> s;
-        load_stencil<double, D>(P, q0, q1, cidx(P, i, j, k), s);
-        double o0, o1;
-        Problem::OperatorCell<double, D>(s, P.tmp1, P.tmp2, P.alpha, o0, o1);
-        const int64_t fc = (int64_t)(i - 1) + (int64_t)(j - 1) * fsy +
-                           (int64_t)(D == 3 ? k - 1 : 0) * fsz;
-        const double r0 = fbase[fc] - o0;
-        const double r1 = fbase[fc + fcomp] - o1;
-        acc += r0 * r0 + r1 * r1;
+  for (int64_t w = (int64_t)blockIdx.x * NORM_WARPS + (threadIdx.x >> 5); w < pieces;
+       w += (int64_t)gridDim.x * NORM_WARPS) {
+    const int64_t chunks = w / nseg;
+    const int seg = (int)(w - chunks * nseg);
+    const int plane = (int)(chunks / nchunk);
+    const int j0 = (int)(chunks - (int64_t)plane * nchunk) * rows + 1;
+    const int j1 = min(j0 + rows - 1, P.n[1]);
+    const int i = seg * 32 + lane + 1, k = D == 3 ? plane + 1 : 0;
+    const int ii = min(i, P.n[0]);  // lanes beyond the row add nothing
+    const double* q0 = static_cast<const double*>(P.q[0]) + cidx(P, ii, j0, k);
+    const double* q1 = static_cast<const double*>(P.q[1]) + cidx(P, ii, j0, k);
+    const double* f = fbase + (int64_t)(ii - 1) + (int64_t)(j0 - 1) * fsy +
+                      (int64_t)(D == 3 ? plane : 0) * fsz;
+    double sum = 0.0;
+    double ps = q0[-P.sy], pc = q0[0], ms = q1[-P.sy], mc = q1[0];
+#pragma unroll 8
+    for (int j = j0; j <= j1; ++j) {
+      Problem::Stencil<double, D> s;
+      s.pc = pc;
+      s.mc = mc;
+      s.pm[0] = q0[-1];
+      s.pp[0] = q0[1];
+      s.mm[0] = q1[-1];
+      s.mp[0] = q1[1];
+      s.pm[1] = ps;
+      s.pp[1] = q0[P.sy];
+      s.mm[1] = ms;
+      s.mp[1] = q1[P.sy];
+      if (D == 3) {
+        s.pm[D - 1] = q0[-P.sz];
+        s.pp[D - 1] = q0[P.sz];
+        s.mm[D - 1] = q1[-P.sz];
+        s.mp[D - 1] = q1[P.sz];
       }
+      double o0, o1;
+      Problem::OperatorCell<double, D>(s, P.tmp1, P.tmp2, P.alpha, o0, o1);
+      const double r0 = f[0] - o0, r1 = f[fcomp] - o1;
+      sum += r0 * r0 + r1 * r1;
+      ps = pc;
+      ms = mc;
+      pc = s.pp[1];
+      mc = s.mp[1];
+      q0 += P.sy;
+      q1 += P.sy;
+      f += fsy;
     }
+    if (i <= P.n[0]) acc += sum;
   }
   const double bs = block_sum(acc);
   double total;
@@ -142,21 +174,25 @@ extern "C" int bsam_gpu_resid_norm_noalloc(int device, int ndims, const int32_t*
     P.tmp1 = dt / h2;
     P.tmp2 = eps * eps / h2;
     const double denom = (double)(2 * n[0] * n[1] * n[2]);
-    // The ticket must start at zero; the partials are written before read.
-    uint32_t* ticket = reinterpret_cast<uint32_t*>(scratch + NOALLOC_MAX_TILES);
-    if (cudaMemsetAsync(ticket, 0, sizeof(uint32_t), s) != cudaSuccess) {
-      rc = BSAM_ERR_CUDA;
-    } else {
-      const dim3 block(32, TILE_Y, 1);
-      const int64_t fsy = n[0], fsz = n[0] * n[1], fcomp = n[0] * n[1] * n[2];
-      if (ndims == 2)
-        k_resid_norm_noalloc<2><<<(unsigned)tiles, block, 0, s>>>(
-            P, f, fsy, fsz, fcomp, (int)tiles_x, (int)tiles_y, scratch, denom, out);
-      else
-        k_resid_norm_noalloc<3><<<(unsigned)tiles, block, 0, s>>>(
-            P, f, fsy, fsz, fcomp, (int)tiles_x, (int)tiles_y, scratch, denom, out);
-      if (cudaGetLastError() != cudaSuccess) rc = BSAM_ERR_CUDA;
-    }
+    // The ticket starts at zero (static storage) and the last CTA of every
+    // launch sets it back; the partials are written before they are read.
+    const int64_t fsy = n[0], fsz = n[0] * n[1], fcomp = n[0] * n[1] * n[2];
+    const int64_t nseg = (n[0] + 31) / 32;
+    // Rows per piece: 16 where that still gives every resident warp one, fewer
+    // (down to a tile's 4) on small patches.
+    constexpr int64_t kCtas = 148 * NORM_CTAS_PER_SM;
+    const int64_t rows = std::max<int64_t>(
+        4, std::min<int64_t>(16, nseg * n[1] * n[2] / (kCtas * NORM_WARPS)));
+    const int64_t nchunk = (n[1] + rows - 1) / rows;
+    const int64_t pieces = nseg * nchunk * n[2];
+    const int64_t ctas = std::min<int64_t>(kCtas, (pieces + NORM_WARPS - 1) / NORM_WARPS);
+    if (ndims == 2)
+      k_resid_norm_noalloc<2><<<(unsigned)ctas, 32 * NORM_WARPS, 0, s>>>(
+          P, f, fsy, fsz, fcomp, (int)nseg, (int)nchunk, (int)rows, pieces, scratch, denom, out);
+    else
+      k_resid_norm_noalloc<3><<<(unsigned)ctas, 32 * NORM_WARPS, 0, s>>>(
+          P, f, fsy, fsz, fcomp, (int)nseg, (int)nchunk, (int)rows, pieces, scratch, denom, out);
+    if (cudaGetLastError() != cudaSuccess) rc = BSAM_ERR_CUDA;
   }
   cudaSetDevice(prev);
   return rc;

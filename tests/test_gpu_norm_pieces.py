@@ -1,0 +1,38 @@
+"""bsam_gpu_resid_norm_noalloc at the edges of a warp's piece (32 columns, 4 to 16
+rows) and of the grid, against the oracle's Operator.  Tolerance: the sums have
+at most 2e5 positive terms, each a few roundings off, added pairwise or in runs
+of at most a few hundred: 1e-12 relative is far above what that can reach."""
+import ctypes
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mx", [(1, 1), (31, 5), (32, 4), (33, 17), (2001, 37), (7, 4000),
+                                (64, 1024), (1, 1, 1), (33, 5, 7), (19, 30, 120), (2, 17, 33)])
+def test_norm_of_ragged_patches(gpu_lib, oracle, mx):
+    import torch
+    nd = len(mx)
+    rng = np.random.default_rng(sum(mx))
+    q = np.asfortranarray(0.5 + 0.1 * rng.standard_normal(tuple(m + 2 for m in mx) + (2,)))
+    f = np.asfortranarray(0.01 * rng.standard_normal(tuple(mx) + (2,)))
+    h, dt, eps, alpha = 1.0 / mx[0], 1e-4, 0.02, 1.0
+    rf = f - oracle.operator(nd, mx, h, dt, alpha, eps, q)
+    total = float(np.sum(rf * rf))
+    qd = torch.from_numpy(q.ravel(order="F").copy()).cuda()
+    fd = torch.from_numpy(f.ravel(order="F").copy()).cuda()
+    m = (ctypes.c_int32 * 3)(*(list(mx) + [1] * (3 - nd)))
+    stream = torch.cuda.current_stream()
+    for _ in range(2):  # the second call finds the ticket the first one left
+        out = torch.full((2,), -1.0, dtype=torch.float64, device="cuda")
+        rc = gpu_lib.bsam_gpu_resid_norm_noalloc(
+            torch.cuda.current_device(), nd, m, h, dt, eps, alpha,
+            ctypes.c_void_p(qd.data_ptr()), ctypes.c_void_p(fd.data_ptr()),
+            ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(stream.cuda_stream))
+        assert rc == 0
+        torch.cuda.synchronize()
+        got = out.cpu().numpy()
+        np.testing.assert_allclose(got[1], total, rtol=1e-12)
+        np.testing.assert_allclose(got[0], np.sqrt(total / (2.0 * np.prod(mx))), rtol=1e-12)
