@@ -316,24 +316,6 @@ __device__ __forceinline__ void setbc_cell(const DevPatch& P, int g0, int g1, in
   }
 }
 
-// The 2D ring cell g of a patch with m1 x m2 interior cells (bottom row, top
-// row, left column, right column).
-__device__ __forceinline__ void ring2(int g, int m1, int m2, int& gi, int& gj) {
-  if (g < m1 + 2) {
-    gi = g;
-    gj = 0;
-  } else if (g < 2 * (m1 + 2)) {
-    gi = g - (m1 + 2);
-    gj = m2 + 1;
-  } else if (g < 2 * (m1 + 2) + m2) {
-    gi = 0;
-    gj = g - 2 * (m1 + 2) + 1;
-  } else {
-    gi = m1 + 1;
-    gj = g - 2 * (m1 + 2) - m2 + 1;
-  }
-}
-
 // SetGhost of a 2D refined level in one launch, one CTA per patch: the
 // patch's coarse-fine interpolation (interp2_ghost on every ring cell), then
 // the sibling copies into its ring (the overlap entries whose dst is this
@@ -387,22 +369,6 @@ static __global__ void k_ghost2(const DevPatch* __restrict__ PT, const int* __re
                          const OverlapCopy* __restrict__ cps, const int2* __restrict__ ranges,
                          int ipass) {
   ghost2_patch(PT, patches[blockIdx.x], cps, ranges[blockIdx.x], ipass);
-}
-
-// The 3D ring cell g of a patch with m1 x m2 x m3 interior cells, in
-// order: the two k planes, then the 2D ring of each interior plane.
-__device__ __forceinline__ void ring3(int g, int m1, int m2, int m3, int& gi, int& gj, int& gk) {
-  const int plane = (m1 + 2) * (m2 + 2), rg2 = 2 * (m1 + 2) + 2 * m2;
-  if (g < 2 * plane) {
-    gk = g < plane ? 0 : m3 + 1;
-    const int r = g % plane;
-    gi = r % (m1 + 2);
-    gj = r / (m1 + 2);
-  } else {
-    const int r0 = g - 2 * plane;
-    gk = 1 + r0 / rg2;
-    ring2(r0 % rg2, m1, m2, gi, gj);
-  }
 }
 
 // SetGhost of a 3D refined level in one launch: k_ghost2's structure with

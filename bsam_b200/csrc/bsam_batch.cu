@@ -1592,10 +1592,14 @@ static int admit(bsam_batch* b, const bsam_batch_problem* prob, const double* q0
       k_init_seeded<3><<<gi, 256, 0, b->stream>>>(b->d_pt, rec0 + S.master, init->seed,
                                                    init->cbar, init->amp, k2);
   }
-  const int64_t total = (int64_t)hcomp;
-  const int nb = (int)((total + 255) / 256);
-  if (nd == 2) k_setbc<double, 2><<<nb, 256, 0, b->stream>>>(b->d_pt, rec0 + S.master, total);
-  else k_setbc<double, 3><<<nb, 256, 0, b->stream>>>(b->d_pt, rec0 + S.master, total);
+  // SetBC takes its patches from a list: the record number, through the staging
+  // ring.
+  int* master = reinterpret_cast<int*>(stage_alloc(b, sizeof(int)));
+  if (!master) return fail(b, BSAM_ERR_NOMEM, "pinned staging allocation failed");
+  *master = rec0 + S.master;
+  const unsigned nb = setbc_blocks(nd, S.cells);
+  if (nd == 2) k_setbc_list<double, 2><<<dim3(nb, 1), SETBC_THREADS, 0, b->stream>>>(b->d_pt, master);
+  else k_setbc_list<double, 3><<<dim3(nb, 1), SETBC_THREADS, 0, b->stream>>>(b->d_pt, master);
   CU(cudaGetLastError());
   SlotState z{SLOT_RUNNING, 0, 0, 0};
   rc = stage_copy(b, b->d_state + s, &z, sizeof(SlotState));
@@ -1739,8 +1743,9 @@ static int admit_many(bsam_batch* b, int n, const bsam_batch_problem* probs,
     k_rows_list<true><<<dim3(gr, na), 256, 0, b->stream>>>(rows);
     CU(cudaEventRecord(b->xin_free, b->stream));
   }
-  if (nd == 2) k_setbc_list<double, 2><<<dim3(gx(maxc), na), 256, 0, b->stream>>>(b->d_pt, masters);
-  else k_setbc_list<double, 3><<<dim3(gx(maxc), na), 256, 0, b->stream>>>(b->d_pt, masters);
+  const dim3 gs(setbc_blocks(nd, maxc), (unsigned)na);
+  if (nd == 2) k_setbc_list<double, 2><<<gs, SETBC_THREADS, 0, b->stream>>>(b->d_pt, masters);
+  else k_setbc_list<double, 3><<<gs, SETBC_THREADS, 0, b->stream>>>(b->d_pt, masters);
   CU(cudaGetLastError());
   stage_commit(b);
   return na;

@@ -75,6 +75,9 @@ struct LevelPlan {
   // Parent of a refined level: its children do not cover it, so the
   // snapshot qs is a full copy of q taken after restriction + SetGhost.
   bool snap = false;
+  CopySpan* d_snap = nullptr;  // the copies of its parent patches
+  int nsnap = 0;
+  int64_t snap_max = 0;
 };
 
 }  // namespace
@@ -126,6 +129,11 @@ struct bsam_gpu {
   CopySpan* d_qold_spans = nullptr;  // CopyQToQold: q -> qold of every patch that has qold
   int nqold_spans = 0;
   int64_t qold_span_max = 0;
+  // SetBC at and below the root: the FP64 state patches, by level (entry l -
+  // minlevel of setbc_first: where level l starts), and the largest one's cells.
+  int* d_setbc = nullptr;
+  std::vector<int> setbc_first;
+  int64_t setbc_cells = 1;
   CopySpan* d_stash_spans = nullptr;
   size_t stash_spans_cap = 0;
   size_t flags_cap = 0;
@@ -165,10 +173,12 @@ struct bsam_gpu {
   double denom = 1.0;        // nrvars * cells of the finest level (ErrorAFAS)
   cudaGraphExec_t step_exec = nullptr;  // V-cycle loop graph (built lazily)
   int graph_kernels_per_vcycle = 0;
-  double* d_trace = nullptr;  // per-V-cycle residuals of the graph path
-  double* h_trace = nullptr;  // pinned
+  // The status and, behind it, the residual of every V-cycle (one copy brings
+  // both back).
   DevStatus* d_status = nullptr;
   DevStatus* h_status = nullptr;  // pinned
+  double* d_trace = nullptr;
+  double* h_trace = nullptr;
   std::vector<double> trace;
   std::string err;
   // instrumentation
@@ -196,6 +206,9 @@ int fail(bsam_gpu* h, int code, const std::string& msg) {
   } while (0)
 
 int64_t roundup(int64_t x, int64_t a) { return (x + a - 1) / a * a; }
+
+size_t status_bytes(int maxvcycles) { return sizeof(DevStatus) + sizeof(double) * maxvcycles; }
+static_assert(sizeof(DevStatus) % sizeof(double) == 0, "the trace follows the status");
 
 LevelPlan& plan(bsam_gpu* h, int level) { return h->levels[level - h->minlevel]; }
 
@@ -320,18 +333,14 @@ void amr_ghost(bsam_gpu* h, int level, int ipass) {
 
 // GetCoarseGhostPoints for the children of a partly covered level: the
 // snapshot qs of every parent patch becomes a full copy of q (taken after
-// restriction and SetGhost).
+// restriction and SetGhost), all of them in one launch (a level of the AMR
+// workload has about 40 such patches: as two copies each they were 80 graph
+// nodes in a row).
 void snapshot(bsam_gpu* h, int level) {
   const LevelPlan& L = plan(h, level);
-  if (!L.snap) return;
-  for (int p : L.patches) {
-    const DevPatch& P = h->hp[p];
-    if (!P.qs[0]) continue;  // not a parent: no child reads a snapshot of it
-    const int64_t lead = 128 / sizeof(double) - 1;
-    for (int c = 0; c < 2; ++c)
-      cudaMemcpyAsync(static_cast<double*>(P.qs[c]) - lead, static_cast<double*>(P.q[c]) - lead,
-                      h->field_elems[p] * sizeof(double), cudaMemcpyDeviceToDevice, h->stream);
-  }
+  if (!L.snap || L.nsnap == 0) return;
+  k_copy_spans<<<copy_spans_grid(L.snap_max, L.nsnap), 256, 0, h->stream>>>(L.d_snap);
+  ++h->stats.launches;
 }
 
 // FillDown(solutionfield) over the refined levels (afas:223-239): each
@@ -544,18 +553,19 @@ int build_step_graph(bsam_gpu* h) {
   return BSAM_OK;
 }
 
-// SetBC on the FP64 state patches of one level.
-int ghost_level(bsam_gpu* h, int level) {
-  for (int p = 0; p < h->nuser; ++p) {
-    const DevPatch& P = h->hp[p];
-    if (P.level != level || P.prec != PREC_F64 || P.delta) continue;
-    int64_t total = (int64_t)(P.n[0] + 2) * (P.n[1] + 2) * (h->rp.ndims == 3 ? P.n[2] + 2 : 1);
-    int nb = (int)((total + 255) / 256);
-    if (h->rp.ndims == 2) k_setbc<double, 2><<<nb, 256, 0, h->stream>>>(h->d_patches, p, total);
-    else k_setbc<double, 3><<<nb, 256, 0, h->stream>>>(h->d_patches, p, total);
-    ++h->stats.launches;
-  }
-  return BSAM_OK;
+// SetBC on the FP64 state patches of the levels from `lo` to `hi` at and below
+// the root, in one launch (each reads and writes only itself).
+void ghost_levels(bsam_gpu* h, int lo, int hi) {
+  const int first = h->setbc_first[std::max(lo, h->minlevel) - h->minlevel];
+  const int last = h->setbc_first[std::min(hi, 0) - h->minlevel + 1];
+  if (last <= first) return;
+  const dim3 g(setbc_blocks(h->rp.ndims, h->setbc_cells), (unsigned)(last - first));
+  const int* list = h->d_setbc + first;
+  if (h->rp.ndims == 2)
+    k_setbc_list<double, 2><<<g, SETBC_THREADS, 0, h->stream>>>(h->d_patches, list);
+  else
+    k_setbc_list<double, 3><<<g, SETBC_THREADS, 0, h->stream>>>(h->d_patches, list);
+  ++h->stats.launches;
 }
 
 int face_rule(int ndims, int face, int code, int* rule) {
@@ -712,12 +722,14 @@ int bsam_gpu_create(bsam_gpu** out, int device, const bsam_run_params* p) {
     return BSAM_ERR_NODEVICE;
   }
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess ||
-      cudaMalloc(&h->d_status, sizeof(DevStatus)) != cudaSuccess ||
-      cudaMallocHost(&h->h_status, sizeof(DevStatus)) != cudaSuccess) {
+      cudaMalloc(&h->d_status, status_bytes(p->maxvcycles)) != cudaSuccess ||
+      cudaMallocHost(&h->h_status, status_bytes(p->maxvcycles)) != cudaSuccess) {
     delete h;
     return BSAM_ERR_CUDA;
   }
   cudaMemset(h->d_status, 0, sizeof(DevStatus));
+  h->d_trace = reinterpret_cast<double*>(h->d_status + 1);
+  h->h_trace = reinterpret_cast<double*>(h->h_status + 1);
   h->d_err = &h->d_status->kerr;
   *out = h;
   return BSAM_OK;
@@ -1100,6 +1112,41 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     }
     h->nqold_spans = (int)spans.size();
   }
+  // SetBC's patches at and below the root, and the snapshots of partly covered
+  // parents (levels >= root below the finest).
+  std::vector<int> setbc_list;
+  h->setbc_first.assign(1, 0);
+  h->setbc_cells = 1;
+  for (int l = minlevel; l <= 0; ++l) {
+    for (int p = 0; p < npatch; ++p) {
+      const DevPatch& P = h->hp[p];
+      if (P.level != l || P.prec != PREC_F64 || P.delta) continue;
+      setbc_list.push_back(p);
+      h->setbc_cells = std::max(h->setbc_cells, cells_of(P.n, nd));
+    }
+    h->setbc_first.push_back((int)setbc_list.size());
+  }
+  if (setbc_list.size() > 65535) return fail(h, BSAM_ERR_ARG, "too many patches below the root");
+  std::vector<CopySpan> snap_spans;
+  std::vector<int> snap_first(h->levels.size() + 1, 0);
+  for (size_t li = 0; li < h->levels.size(); ++li) {
+    LevelPlan& L = h->levels[li];
+    snap_first[li] = (int)snap_spans.size();
+    L.snap_max = 0;
+    if (L.level >= 0 && L.level < finestlevel)
+      for (int p : L.patches) {
+        const DevPatch& P = h->hp[p];
+        if (!P.qs[0]) continue;  // not a parent: no child reads a snapshot of it
+        const int64_t lead = 128 / sizeof(double) - 1;
+        for (int c = 0; c < 2; ++c)
+          snap_spans.push_back(CopySpan{static_cast<const double*>(P.q[c]) - lead,
+                                        static_cast<double*>(P.qs[c]) - lead,
+                                        h->field_elems[p]});
+        L.snap_max = std::max(L.snap_max, h->field_elems[p]);
+      }
+    L.nsnap = (int)snap_spans.size() - snap_first[li];
+    if (L.nsnap > 65535) return fail(h, BSAM_ERR_ARG, "too many parent patches on a level");
+  }
   // Parents of the twins are the masters' parents.
   for (int r = npatch; r < nrec; ++r) h->hp[r].parent = h->hp[rec_src[r]].parent;
   for (int r = 0; r < nrec; ++r)
@@ -1273,10 +1320,6 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
                             (int)Fused3<float>::SMEM));
     h->attrs_set = true;
   }
-  // The residual trace buffers live as long as the handle (maxvcycles is
-  // fixed at creation).
-  if (!h->d_trace) CU(cudaMalloc(&h->d_trace, sizeof(double) * h->rp.maxvcycles));
-  if (!h->h_trace) CU(cudaMallocHost(&h->h_trace, sizeof(double) * h->rp.maxvcycles));
   {
     int64_t ncells = 0;
     for (int p : h->masters) ncells += cells_of(h->hp[p].n, nd);
@@ -1315,6 +1358,8 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     const size_t o_ovl_dst = place(sizeof(OverlapCopy) * ovl_by_dst.size());
     const size_t o_ovl_rng = place(sizeof(int2) * ovl_range.size());
     const size_t o_qold = place(sizeof(CopySpan) * qold_spans.size());
+    const size_t o_snap = place(sizeof(CopySpan) * snap_spans.size());
+    const size_t o_setbc = place(sizeof(int) * setbc_list.size());
     const size_t o_maps = place(sizeof(CUtensorMap) * maps.size());
     const size_t o_chains = place(sizeof(ChainPlan) * plans.size());
     const size_t o_part = place(sizeof(double) * h->max_items);
@@ -1333,6 +1378,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     h->d_plist = plist_all.empty() ? nullptr : reinterpret_cast<int*>(base + o_plist);
     h->d_ovl = ovl_all.empty() ? nullptr : reinterpret_cast<OverlapCopy*>(base + o_ovl);
     h->d_qold_spans = qold_spans.empty() ? nullptr : reinterpret_cast<CopySpan*>(base + o_qold);
+    h->d_setbc = reinterpret_cast<int*>(base + o_setbc);
     h->d_tmaps = maps.empty() ? nullptr : reinterpret_cast<CUtensorMap*>(base + o_maps);
     h->d_chains = plans.empty() ? nullptr : reinterpret_cast<ChainPlan*>(base + o_chains);
     h->d_partials = reinterpret_cast<double*>(base + o_part);
@@ -1342,6 +1388,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
       LevelPlan& L = h->levels[li];
       L.d_plist = h->d_plist ? h->d_plist + span_plist[li].first : nullptr;
       L.d_ovl = h->d_ovl ? h->d_ovl + span_ovl[li].first : nullptr;
+      L.d_snap = reinterpret_cast<CopySpan*>(base + o_snap) + snap_first[li];
       L.d_ovl_by_dst = ovl_by_dst.empty()
                            ? nullptr
                            : reinterpret_cast<OverlapCopy*>(base + o_ovl_dst) + span_ovl[li].first;
@@ -1367,6 +1414,8 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     put(o_ovl_dst, ovl_by_dst.data(), sizeof(OverlapCopy) * ovl_by_dst.size());
     put(o_ovl_rng, ovl_range.data(), sizeof(int2) * ovl_range.size());
     put(o_qold, qold_spans.data(), sizeof(CopySpan) * qold_spans.size());
+    put(o_snap, snap_spans.data(), sizeof(CopySpan) * snap_spans.size());
+    put(o_setbc, setbc_list.data(), sizeof(int) * setbc_list.size());
     put(o_maps, maps.data(), sizeof(CUtensorMap) * maps.size());
     put(o_chains, plans.data(), sizeof(ChainPlan) * plans.size());
     const int urc = h2d_bounce(h, h->d_meta, img.data(), img.size());
@@ -1452,12 +1501,9 @@ int bsam_gpu_set_ghost(bsam_gpu* h) {
   if (!h || !h->have_hierarchy) return BSAM_ERR_STATE;
   CU(cudaSetDevice(h->device));
   // Coarse levels first: a refined level's interpolation reads its parent.
-  for (int l = h->minlevel; l <= h->finestlevel; ++l) {
-    if (plan(h, l).amr) amr_ghost(h, l, 0);
-    else ghost_level(h, l);
-  }
+  ghost_levels(h, h->minlevel, 0);
+  for (int l = 1; l <= h->finestlevel; ++l) amr_ghost(h, l, 0);
   CU(cudaGetLastError());
-  CU(cudaStreamSynchronize(h->stream));
   return BSAM_OK;
 }
 
@@ -1467,9 +1513,8 @@ int bsam_gpu_set_ghost_level(bsam_gpu* h, int level) {
     return fail(h, BSAM_ERR_ARG, "set_ghost_level: level out of range");
   CU(cudaSetDevice(h->device));
   if (plan(h, level).amr) amr_ghost(h, level, 0);
-  else ghost_level(h, level);
+  else ghost_levels(h, level, level);
   CU(cudaGetLastError());
-  CU(cudaStreamSynchronize(h->stream));
   return BSAM_OK;
 }
 
@@ -1478,7 +1523,6 @@ int bsam_gpu_fill_down(bsam_gpu* h) {
   CU(cudaSetDevice(h->device));
   if (h->amr) filldown(h);
   CU(cudaGetLastError());
-  CU(cudaStreamSynchronize(h->stream));
   return BSAM_OK;
 }
 
@@ -1495,7 +1539,6 @@ int bsam_gpu_restrict_level(bsam_gpu* h, int level) {
   ++h->stats.launches;
   amr_ghost(h, level - 1, 0);
   CU(cudaGetLastError());
-  CU(cudaStreamSynchronize(h->stream));
   return BSAM_OK;
 }
 
@@ -1504,8 +1547,8 @@ int bsam_gpu_copy_q_to_qold(bsam_gpu* h) {
   CU(cudaSetDevice(h->device));
   // qold exists on levels >= root only (Source reads it there).
   if (h->nqold_spans == 0) return BSAM_OK;
-  const int bx = (int)std::min<int64_t>((h->qold_span_max + 255) / 256, 64);
-  k_copy_spans<<<dim3(bx, h->nqold_spans), 256, 0, h->stream>>>(h->d_qold_spans);
+  k_copy_spans<<<copy_spans_grid(h->qold_span_max, h->nqold_spans), 256, 0, h->stream>>>(
+      h->d_qold_spans);
   ++h->stats.launches;
   CU(cudaGetLastError());
   return BSAM_OK;
@@ -1549,9 +1592,7 @@ int bsam_gpu_multigrid_iterations(bsam_gpu* h, int* nvcycles, double* residual, 
       CU(cudaGraphLaunch(h->step_exec, h->stream));
       ++h->stats.launches;
     }
-    CU(cudaMemcpyAsync(h->h_status, h->d_status, sizeof(DevStatus), cudaMemcpyDeviceToHost,
-                       h->stream));
-    CU(cudaMemcpyAsync(h->h_trace, h->d_trace, sizeof(double) * h->rp.maxvcycles,
+    CU(cudaMemcpyAsync(h->h_status, h->d_status, status_bytes(h->rp.maxvcycles),
                        cudaMemcpyDeviceToHost, h->stream));
     CU(cudaStreamSynchronize(h->stream));
     it = std::max(1, std::min(h->h_status->iters, h->rp.maxvcycles));
@@ -2010,8 +2051,8 @@ int bsam_gpu_stash(bsam_gpu* h) {
     const int urc = h2d_bounce(h, h->d_stash_spans, spans.data(), sizeof(CopySpan) * spans.size());
     if (urc) return urc;
   }
-  const int bx = (int)std::min<int64_t>((span_max + 255) / 256, 64);
-  k_copy_spans<<<dim3(bx, (unsigned)spans.size()), 256, 0, h->stream>>>(h->d_stash_spans);
+  k_copy_spans<<<copy_spans_grid(span_max, (int64_t)spans.size()), 256, 0, h->stream>>>(
+      h->d_stash_spans);
   ++h->stats.launches;
   CU(cudaGetLastError());
   // The span list is host memory: wait until it has been read.
@@ -2140,7 +2181,7 @@ int bsam_gpu_regrid(bsam_gpu* h, int npatch, const bsam_patch_desc* patches, int
     }
     const auto grid_x = [](int64_t n) { return (unsigned)std::min<int64_t>((n + 255) / 256, 64); };
     if (e == cudaSuccess && !spans.empty()) {
-      k_copy_spans<<<dim3(grid_x(span_max), (unsigned)spans.size()), 256, 0, h->stream>>>(
+      k_copy_spans<<<copy_spans_grid(span_max, (int64_t)spans.size()), 256, 0, h->stream>>>(
           reinterpret_cast<const CopySpan*>(h->d_regrid + o_sp));
       ++h->stats.launches;
       e = cudaGetLastError();
@@ -2229,8 +2270,6 @@ int bsam_gpu_destroy(bsam_gpu* h) {
     cudaEventDestroy(e.second);
   }
   free_hierarchy(h);
-  if (h->d_trace) cudaFree(h->d_trace);
-  if (h->h_trace) cudaFreeHost(h->h_trace);
   if (h->h_pin) cudaFreeHost(h->h_pin);
   if (h->spare_arena) cudaFree(h->spare_arena);
   if (h->d_stash) cudaFree(h->d_stash);
