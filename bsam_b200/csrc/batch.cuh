@@ -18,6 +18,7 @@
 #include "bottom.cuh"
 #include "kernels.cuh"
 #include "mixed.cuh"
+#include "rows.cuh"
 
 namespace bsam {
 
@@ -554,39 +555,6 @@ __global__ void k_init_seeded_list(const DevPatch* __restrict__ PT,
   init_seeded_range<D>(P, t.seed, t.cbar, t.amp, t.k2,
                        (int64_t)blockIdx.x * blockDim.x + threadIdx.x,
                        (int64_t)gridDim.x * blockDim.x);
-}
-
-// One problem's root state between the caller's Fortran-ordered q (both
-// components, ghosts included: `rows` rows of e0 values per component) and
-// the pitched master fields q0, q1 (row pitch sy; in 3D the plane pitch is
-// sy * (n1 + 2), so the rows of every plane follow each other at pitch sy).
-// The packed copy lives in the engine's device transfer buffer, which one
-// contiguous DMA per problem fills from, or empties into, the caller's
-// buffer: pitched host copies of rows this short run far below the link's
-// speed.
-struct RowsTask {
-  double* packed;
-  double* q[2];
-  int64_t rows, sy;
-  int32_t e0, pad_;
-};
-
-// A warp per row: packed -> pitched (unpack) or pitched -> packed (pack).
-template <bool UNPACK>
-__global__ void __launch_bounds__(256) k_rows_list(const RowsTask* __restrict__ tasks) {
-  const RowsTask t = tasks[blockIdx.y];
-  const int lane = threadIdx.x & 31;
-  const int64_t wpb = blockDim.x >> 5;
-  for (int64_t r = (int64_t)blockIdx.x * wpb + (threadIdx.x >> 5); r < 2 * t.rows;
-       r += (int64_t)gridDim.x * wpb) {
-    const int c = r >= t.rows ? 1 : 0;
-    double* pitched = t.q[c] + (r - c * t.rows) * t.sy;
-    double* packed = t.packed + r * t.e0;
-    for (int i = lane; i < t.e0; i += 32) {
-      if (UNPACK) pitched[i] = packed[i];
-      else packed[i] = pitched[i];
-    }
-  }
 }
 
 __global__ void k_batch_budget(BatchCtl* __restrict__ ctl, int ticks) {

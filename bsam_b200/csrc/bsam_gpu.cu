@@ -20,12 +20,14 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
 #include <map>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include "../../include/bsam_gpu.h"
@@ -36,6 +38,7 @@
 #include "mixed.cuh"
 #include "amr.cuh"
 #include "regrid.cuh"
+#include "rows.cuh"
 #include "stats.cuh"
 #include "engine_view.h"
 
@@ -122,6 +125,8 @@ struct bsam_gpu {
   // before the buffer is written again.
   void* h_pin = nullptr;
   size_t pin_cap = 0;
+  bool pin_busy = false;       // queued work still reads it (a put_field)
+  cudaEvent_t slot_ev[8] = {};  // put / get of large fields: a piece's slot is free / full
   bool attrs_set = false;      // the fused kernels' shared-memory attributes
   uint8_t* d_flags = nullptr;  // bsam_gpu_errflags_level's device flags
   int32_t* d_sat = nullptr;    // bsam_gpu_tag_level's summed-area tables
@@ -217,6 +222,10 @@ LevelPlan& plan(bsam_gpu* h, int level) { return h->levels[level - h->minlevel];
 // through the driver's staging, which handles regridding side by side on
 // several host threads contend for.
 void* pin_reserve(bsam_gpu* h, size_t bytes) {
+  if (h->pin_busy) {
+    cudaStreamSynchronize(h->stream);
+    h->pin_busy = false;
+  }
   if (bytes > h->pin_cap) {
     if (h->h_pin) cudaFreeHost(h->h_pin);
     h->h_pin = nullptr;
@@ -682,6 +691,71 @@ int engine_device(bsam_gpu* h) { return h ? h->device : -1; }
 
 }  // namespace bsam
 
+namespace {
+
+// put_field / get_field of q or qold (both components, ghost ring included)
+// between the caller's pageable array and the pitched fields, through
+// page-locked memory: a kernel spreads the rows from it, or packs them into it,
+// over the bus; a host copy does the rest.  For small fields, in the bounce
+// buffer, that is one launch instead of two staged pitched copies (a 16 KB
+// field: put 28 -> 12 us, get 27 -> 19).  Large fields go in pieces that a few
+// host threads copy side by side, each through two slots of its own, so that
+// host copies and the bus overlap (128^3, 35 MB: put 3.9 -> 1.2 ms, get 1.9 ->
+// 1.5).  Between the two limits the driver's pitched copies are as good (512^2,
+// 4 MB: 0.30 ms up and 0.28 down, 0.24 and 0.27 in pieces) and need no
+// page-locked memory, which costs 1 ms per MB to allocate.
+constexpr size_t kBounceBytes = (size_t)128 << 10;
+constexpr size_t kThreadedBytes = (size_t)8 << 20;
+constexpr size_t kPieceBytes = (size_t)512 << 10;
+constexpr int kCopyThreads = 4;
+constexpr size_t kPieceBlock = 2 * kCopyThreads * kPieceBytes;  // the slots of one copy
+
+// The page-locked blocks of large copies, for all handles of the process: a
+// copy takes one and gives it back when it is done with it; up to two wait for
+// the next copies, until the last handle is destroyed.
+struct PieceBlocks {
+  std::mutex mutex;
+  std::vector<void*> idle;
+  int handles = 0;
+  static PieceBlocks& get() {
+    static PieceBlocks* p = new PieceBlocks;  // outlives every handle
+    return *p;
+  }
+  void* take() {
+    {
+      std::lock_guard<std::mutex> lock(mutex);
+      if (!idle.empty()) {
+        void* p = idle.back();
+        idle.pop_back();
+        return p;
+      }
+    }
+    void* p = nullptr;
+    return cudaHostAlloc(&p, kPieceBlock, cudaHostAllocPortable) == cudaSuccess ? p : nullptr;
+  }
+  void give(void* p) {
+    {
+      std::lock_guard<std::mutex> lock(mutex);
+      if (handles > 0 && idle.size() < 2) {
+        idle.push_back(p);
+        return;
+      }
+    }
+    cudaFreeHost(p);
+  }
+  void count(int d) {
+    std::vector<void*> drop;
+    {
+      std::lock_guard<std::mutex> lock(mutex);
+      handles += d;
+      if (handles == 0) drop.swap(idle);
+    }
+    for (void* p : drop) cudaFreeHost(p);
+  }
+};
+
+}  // namespace
+
 extern "C" {
 
 const char* bsam_gpu_strerror(int code) {
@@ -731,6 +805,7 @@ int bsam_gpu_create(bsam_gpu** out, int device, const bsam_run_params* p) {
   h->d_trace = reinterpret_cast<double*>(h->d_status + 1);
   h->h_trace = reinterpret_cast<double*>(h->h_status + 1);
   h->d_err = &h->d_status->kerr;
+  PieceBlocks::get().count(1);
   *out = h;
   return BSAM_OK;
 }
@@ -1442,6 +1517,87 @@ static int field_ptr(bsam_gpu* h, int patch, int field, int comp, double** ptr, 
   return BSAM_OK;
 }
 
+static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir) {
+  const int64_t rows = 2 * task.rows;
+  const size_t row_bytes = sizeof(double) * task.e0;
+  auto launch = [&](double* packed, int64_t r0, int64_t r1) {
+    RowsTask t = task;
+    t.packed = packed - r0 * task.e0;  // so that row r0 lies at `packed`
+    const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((r1 - r0 + 7) / 8, 592));
+    if (dir == 0) k_rows<true><<<g, 256, 0, h->stream>>>(t, r0, r1);
+    else k_rows<false><<<g, 256, 0, h->stream>>>(t, r0, r1);
+    return cudaGetLastError();
+  };
+  if (row_bytes * rows <= kBounceBytes) {
+    double* pin = static_cast<double*>(pin_reserve(h, row_bytes * rows));
+    if (!pin) return fail(h, BSAM_ERR_NOMEM, "page-locked staging allocation failed");
+    if (dir == 0) std::memcpy(pin, host, row_bytes * rows);
+    CU(launch(pin, 0, rows));
+    ++h->stats.launches;
+    if (dir == 0) {
+      h->pin_busy = true;
+    } else {
+      CU(cudaStreamSynchronize(h->stream));
+      std::memcpy(host, pin, row_bytes * rows);
+    }
+    return BSAM_OK;
+  }
+  const int64_t per = (int64_t)(kPieceBytes / row_bytes);
+  const int64_t pieces = (rows + per - 1) / per;
+  for (cudaEvent_t& e : h->slot_ev)
+    if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+  char* pin = static_cast<char*>(PieceBlocks::get().take());
+  if (!pin) return fail(h, BSAM_ERR_NOMEM, "page-locked staging allocation failed");
+  const int nt = (int)std::max(1u, std::min((unsigned)kCopyThreads,
+                                            std::thread::hardware_concurrency()));
+  std::atomic<int> failed{(int)cudaSuccess};
+  // Thread t takes pieces t, t + nt, ..., the k-th of them in its slot k % 2.
+  auto work = [&](int t) {
+    cudaError_t e = cudaSetDevice(h->device);
+    auto first = [&](int64_t k) { return (t + k * nt) * per; };
+    auto last = [&](int64_t k) { return std::min(rows, first(k) + per); };
+    auto buf = [&](int64_t k) {
+      return reinterpret_cast<double*>(pin + (2 * t + (int)(k & 1)) * kPieceBytes);
+    };
+    auto ev = [&](int64_t k) { return h->slot_ev[2 * t + (int)(k & 1)]; };
+    const int64_t n = (pieces - t + nt - 1) / nt;
+    auto issue = [&](int64_t k) {
+      if (e == cudaSuccess) e = launch(buf(k), first(k), last(k));
+      if (e == cudaSuccess) e = cudaEventRecord(ev(k), h->stream);
+    };
+    if (dir != 0)
+      for (int64_t k = 0; k < std::min<int64_t>(2, n); ++k) issue(k);
+    for (int64_t k = 0; k < n && e == cudaSuccess; ++k) {
+      double* user = host + first(k) * task.e0;
+      const size_t bytes = row_bytes * (size_t)(last(k) - first(k));
+      if (dir == 0) {
+        if (k >= 2) e = cudaEventSynchronize(ev(k));
+        if (e != cudaSuccess) break;
+        std::memcpy(buf(k), user, bytes);
+        issue(k);
+      } else {
+        e = cudaEventSynchronize(ev(k));
+        if (e != cudaSuccess) break;
+        std::memcpy(user, buf(k), bytes);
+        if (k + 2 < n) issue(k + 2);
+      }
+    }
+    if (e != cudaSuccess) failed.store((int)e);
+  };
+  std::vector<std::thread> pool;
+  for (int t = 1; t < nt; ++t) pool.emplace_back(work, t);
+  work(0);
+  for (auto& t : pool) t.join();
+  h->stats.launches += pieces;
+  const cudaError_t done = cudaStreamSynchronize(h->stream);  // the block's next user may write it
+  if (done != cudaSuccess) failed.store((int)done);
+  PieceBlocks::get().give(pin);
+  if (failed.load() != (int)cudaSuccess)
+    return fail(h, BSAM_ERR_CUDA,
+                std::string("field copy: ") + cudaGetErrorString((cudaError_t)failed.load()));
+  return BSAM_OK;
+}
+
 // Copy between a Fortran array and the pitched device field; dir 0 = H2D.
 static int copy_field(bsam_gpu* h, int patch, int field, double* host, int dir) {
   if (!h || !h->have_hierarchy) return BSAM_ERR_STATE;
@@ -1462,7 +1618,16 @@ static int copy_field(bsam_gpu* h, int patch, int field, double* host, int dir) 
     double* hbase = host + comp * hcomp;
     if (g == 1) {
       // With the ghost ring every row of every plane sits at stride sy on the
-      // device (sz = sy * (n1 + 2)): one pitched copy per component.
+      // device (sz = sy * (n1 + 2)).
+      const size_t bytes = 2 * hcomp * sizeof(double);
+      const bool pieces = bytes >= kThreadedBytes && e0 * sizeof(double) <= kPieceBytes;
+      if (bytes <= kBounceBytes || pieces) {
+        double* dev1;
+        const int rc1 = field_ptr(h, patch, field, 1, &dev1, &interior);
+        if (rc1) return fail(h, rc1, "field not held for this patch");
+        return copy_state(h, RowsTask{nullptr, {dev, dev1}, (int64_t)e1 * e2, P.sy, e0, 0}, host,
+                          dir);
+      }
       if (dir == 0)
         CU(cudaMemcpy2DAsync(dev, P.sy * sizeof(double), hbase, e0 * sizeof(double),
                              e0 * sizeof(double), (size_t)e1 * e2, cudaMemcpyHostToDevice,
@@ -2271,6 +2436,8 @@ int bsam_gpu_destroy(bsam_gpu* h) {
   }
   free_hierarchy(h);
   if (h->h_pin) cudaFreeHost(h->h_pin);
+  for (cudaEvent_t e : h->slot_ev)
+    if (e) cudaEventDestroy(e);
   if (h->spare_arena) cudaFree(h->spare_arena);
   if (h->d_stash) cudaFree(h->d_stash);
   if (h->d_stash_spans) cudaFree(h->d_stash_spans);
@@ -2282,6 +2449,7 @@ int bsam_gpu_destroy(bsam_gpu* h) {
   if (h->h_status) cudaFreeHost(h->h_status);
   if (h->stream) cudaStreamDestroy(h->stream);
   delete h;
+  PieceBlocks::get().count(-1);
   return BSAM_OK;
 }
 

@@ -1,0 +1,39 @@
+"""put_field / get_field round trips at the edges of the copy paths (the bounce
+buffer up to 128 KiB, the driver's pitched copies, pieces copied by several host
+threads from 8 MiB), in 2D and 3D, and twice in a row from one array."""
+import numpy as np
+import pytest
+
+import bsam_b200 as B
+from bsam_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("mx", [(2, 2), (34, 6), (88, 88), (88, 90), (256, 256), (720, 724), (722, 724),
+                                (1022, 512),
+                                (2, 2, 2), (62, 30, 14), (64, 64, 128), (100, 70, 76)])
+def test_fields_come_back_as_put(gpu_lib, mx):
+    nd = len(mx)
+    rng = np.random.default_rng(sum(mx))
+    h = 1.0 / mx[0]
+    prob = W.Problem(ndims=nd, mx=tuple(mx) + (1,) * (3 - nd), eps=0.02, dt=1e-4, nsteps=1,
+                     qerrortol=1e-8, xupper=tuple([n * h for n in mx] + [1.0] * (3 - nd)),
+                     c0=np.full(int(np.prod(mx)), 0.5))
+    shape = tuple(m + 2 for m in mx) + (2,)
+    a = np.asfortranarray(rng.standard_normal(shape))
+    b = np.asfortranarray(rng.standard_normal(shape))
+    out = np.empty(shape, order="F")
+    with B.Solver(prob) as s:
+        s.put_q(a)
+        s.get_q_into(out)
+        assert np.array_equal(out, a)
+        work = a.copy(order="F")
+        s.put_q(work)
+        work[...] = b  # the array is the caller's again once put returns
+        s.get_q_into(out)
+        assert np.array_equal(out, a)
+        s.put_q(a)
+        s.put_q(b)
+        s.get_q_into(out)
+        assert np.array_equal(out, b)
