@@ -34,6 +34,7 @@
 #include "bsam_types.h"
 #include "kernels.cuh"
 #include "smooth_fused.cuh"
+#include "stage2.cuh"
 #include "chain.cuh"
 #include "mixed.cuh"
 #include "amr.cuh"
@@ -52,6 +53,9 @@ constexpr int64_t MIXED_FP64_CELLS = 4096;
 // (levels above it may run them), per dimensionality.
 constexpr int FUSED_BOTTOM_CELLS_2D = 1024;
 constexpr int FUSED_BOTTOM_CELLS_3D = 512;
+// Largest level of the bottom chain where other levels run above it.
+constexpr int64_t CHAIN_TOP_CELLS_2D = 128 * 128;
+constexpr int64_t CHAIN_TOP_CELLS_3D = 8192;
 
 struct LevelPlan {
   int level = 0;
@@ -375,12 +379,41 @@ void launch_transfer_d(bsam_gpu* h, const LevelPlan& L, int pc, int pp, int what
   else launch_transfer_t<double, double, D>(h, L, what);
 }
 
+// A 2D level's stage with its transfer (stage2.cuh).  Tiles of 32 x 16 where
+// they give every SM two (V-cycle of 512^2 FP64 137 us against 140 with 32 x 8,
+// of 1024^2 280 against 302), of 32 x 8 on smaller levels (160^2 78 against 82,
+// 256^2 100 against 102).
+template <class T, bool DELTA>
+void launch_stage2_t(bsam_gpu* h, const LevelPlan& L, int dir) {
+  const int p = L.patches[0];
+  const DevPatch& P = h->hp[p];
+  const unsigned tx = (unsigned)(P.n[0] + 31) / 32;
+  const int upd = dir == 1 && P.master >= 0, nu = h->rp.nsmoothingpasses;
+  auto tiles = [&](auto ty) {
+    using S = Stage2<T, DELTA, decltype(ty)::value>;
+    k_stage2<T, DELTA, decltype(ty)::value>
+        <<<dim3(tx, (unsigned)(P.n[1] + S::TY - 1) / S::TY), S::THREADS, S::SMEM, h->stream>>>(
+            h->d_patches, p, dir, nu, upd);
+  };
+  if (tx * ((unsigned)(P.n[1] + 15) / 16) >= 2 * 148) tiles(std::integral_constant<int, 16>{});
+  else tiles(std::integral_constant<int, 8>{});
+  ++h->stats.launches;
+}
+
+void launch_stage2(bsam_gpu* h, const LevelPlan& L, int dir) {
+  if (!h->mixed) launch_stage2_t<double, false>(h, L, dir);
+  else if (L.prec == PREC_F32) launch_stage2_t<float, true>(h, L, dir);
+  else launch_stage2_t<double, true>(h, L, dir);
+}
+
 // LevelRelax (afas:523-547).  dir selects the buffers of a fused level:
 // 0 = pre-smoothing (q -> qb), 1 = post-smoothing (qb -> q).
 void relax_level(bsam_gpu* h, int level, int dir) {
   const LevelPlan& L = plan(h, level);
   stage_begin(h, level);
-  if (L.fused) {
+  if (L.fused && h->rp.ndims == 2) {
+    launch_stage2(h, L, dir);
+  } else if (L.fused) {
     if (L.prec == PREC_F32)
       k_smooth3_fused<float><<<L.nfused, Fused3<float>::THREADS, Fused3<float>::SMEM, h->stream>>>(
           h->d_patches, L.d_fused, dir, 0, h->d_err);
@@ -416,13 +449,15 @@ void transfer(bsam_gpu* h, int level, int what) {
     else launch_transfer_d<3>(h, L, L.prec, pp, w);
     ++h->stats.launches;
   };
+  // A 2D fused level's stages restrict and correct it themselves.
+  const bool in_stage = L.fused && h->rp.ndims == 2;
   if (what == 0) {
-    launch(0);
+    if (!in_stage) launch(0);
     amr_ghost(h, level - 1, 0);
     snapshot(h, level - 1);
     launch(2);
   } else {
-    launch(1);
+    if (!in_stage) launch(1);
     amr_ghost(h, level, 0);
   }
 }
@@ -514,7 +549,8 @@ void launch_update(bsam_gpu* h) {
 // One outer iteration of MultigridIterations: V-cycle, then ErrorAFAS.
 void iteration(bsam_gpu* h) {
   vcycle(h, h->finestlevel);
-  if (h->mixed) launch_update(h);
+  // A 2D fused finest level has updated its master in its last stage.
+  if (h->mixed && !(h->rp.ndims == 2 && plan(h, h->finestlevel).fused)) launch_update(h);
   if (h->amr) filldown(h);  // FillDown(solutionfield) after the V-cycle (afas:73)
   launch_resid(h);
 }
@@ -951,10 +987,18 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
   const int64_t fp64_cells = h->tuning.bottom_cells > 0 ? h->tuning.bottom_cells
                                                         : MIXED_FP64_CELLS;
   // Bottom level: the finest level from which every chain of levels down to
-  // the coarsest fits in the shared memory of one cluster (chain.cuh).  A
-  // pass costs less there than a launch per pass at every size that fits
-  // (128^2 FP64: 0.5 against 5.3 us; 32^3: 1.0 against 6.0 us), so the
-  // largest that fits is taken, within the caller's bottom_cells if given.
+  // the coarsest fits in the shared memory of one cluster (chain.cuh) and pays
+  // there.  A whole FP64 problem that fits does: its V-cycle loop runs in the
+  // one launch (192^2 V-cycle 70 us, against 85 with its finest level as
+  // stages).  Below other levels a chain's top level has 16 SMs against all of
+  // them: in 2D a level of 128^2 still costs less in the chain (256^2 FP64 97
+  // against 102 us a V-cycle, 256^2 mixed 107 against 113) and one of 192^2 or
+  // 256^2 less as stages (512^2 mixed 140 against 160 us); in 3D a level of
+  // 16^3 (64^3 FP64 181 against 197 us) or 24 x 16 x 20 (96 x 64 x 80 mixed 218
+  // against 235) costs less in the chain and one of 32^3 less as launches (64^3
+  // 181 against 191, 128^3 491 against 505).  A caller's bottom_cells stands as
+  // given.
+  const int64_t chain_top = nd == 3 ? CHAIN_TOP_CELLS_3D : CHAIN_TOP_CELLS_2D;
   int64_t bmax = dflt ? INT64_MAX : h->tuning.bottom_cells;
   if (dflt && h->tuning.fuse_smoother != 0)
     bmax = nd == 3 ? FUSED_BOTTOM_CELLS_3D : FUSED_BOTTOM_CELLS_2D;
@@ -966,7 +1010,8 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
   std::vector<ChainPlan> plans;
   for (int l = std::min(finestlevel, 0); bmax > 0 && l >= minlevel; --l) {
     const bool loop = l == finestlevel && !h->mixed && finestlevel == 0;
-    if (find_chains(h, npatch, patches, l, bmax, fp64_cells, loop, chains, plans)) {
+    const int64_t cells = loop || !dflt ? bmax : std::min(bmax, chain_top);
+    if (find_chains(h, npatch, patches, l, cells, fp64_cells, loop, chains, plans)) {
       h->bottom_level = l;
       h->chain_loop = loop && chains.size() == 1;
       break;
@@ -991,6 +1036,14 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     if (twin_of[p] >= 0) rec_src[twin_of[p]] = p;
   }
 
+  // Levels of a single patch.
+  std::vector<char> alone(finestlevel - minlevel + 1, 0);
+  for (int p = 0; p < npatch; ++p)
+    if (patches[p].level >= minlevel && patches[p].level <= finestlevel) {
+      char& n = alone[patches[p].level - minlevel];
+      n = n == 0 ? 1 : 2;
+    }
+  for (char& n : alone) n = n == 1;
   const double eps2 = h->rp.eps * h->rp.eps;
   size_t total = 0;
   std::vector<size_t> offs(nrec);
@@ -1077,18 +1130,21 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     if (P.delta)
       for (int f = 0; f < 2 * nd; ++f)
         if (P.bc[f] == BC_REFLECT) P.bc[f] = BC_NEGATE;
-    // Fused stages: 3D V-cycle levels with a parent above the bottom, all
-    // faces physical (the stage derives face ghosts from the tile itself).
+    // Fused stages: V-cycle levels of uniform hierarchies (in 2D also the root
+    // of a refined one and the levels below it) with a parent, above the bottom
+    // chain.  3D, on request: all faces physical (the stage derives face ghosts
+    // from the tile itself).  2D, unless the caller wants every level as launches
+    // (bottom_cells -1): one patch, at most two sweeps (the tile's halo of 4).
     const int fmin = std::max(8, h->tuning.fuse_min_n);
     bool periodic = false;
     for (int f = 0; f < 2 * nd; ++f) periodic |= P.bc[f] == BC_PERIODIC;
-    P.fused = (h->tuning.fuse_smoother != 0 && nd == 3 && finestlevel == 0 && in_vcycle &&
-               d.parent >= 0 && !periodic &&
-               d.level > h->bottom_level && !(P.delta && P.prec == PREC_F64) &&
-               P.n[0] >= fmin && P.n[1] >= fmin && P.n[2] >= fmin)
-                  ? 1
-                  : 0;
-    if (P.fused) {
+    const bool fuse3 = h->tuning.fuse_smoother != 0 && nd == 3 && finestlevel == 0 && !periodic &&
+                       !(P.delta && P.prec == PREC_F64) && P.n[0] >= fmin && P.n[1] >= fmin &&
+                       P.n[2] >= fmin;
+    const bool fuse2 = nd == 2 && h->tuning.bottom_cells >= 0 && d.level <= 0 &&
+                       h->rp.nsmoothingpasses <= 2 && alone[d.level - minlevel];
+    P.fused = (fuse3 || fuse2) && in_vcycle && d.parent >= 0 && d.level > h->bottom_level ? 1 : 0;
+    if (P.fused && nd == 3) {
       const int ftx = P.prec == PREC_F32 ? Fused3<float>::TX : Fused3<double>::TX;
       const int fty = P.prec == PREC_F32 ? Fused3<float>::TY : Fused3<double>::TY;
       const int tiles = ((P.n[0] + ftx - 1) / ftx) * ((P.n[1] + fty - 1) / fty);
@@ -1231,7 +1287,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
   std::vector<CUtensorMap> maps;
   {
     for (int r = 0; r < nrec; ++r)
-      if (h->hp[r].fused) fused_recs.push_back(r);
+      if (h->hp[r].fused && nd == 3) fused_recs.push_back(r);
     if (!fused_recs.empty()) {
       maps.resize(7 * fused_recs.size());
       for (size_t k = 0; k < fused_recs.size(); ++k) {
@@ -1271,7 +1327,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     if (!L.fused)
       for (int p : L.patches) h->hp[p].fused = 0;
     s = (int)all.size();
-    if (L.fused)
+    if (L.fused && nd == 3)
       for (int p : L.patches) {
         const DevPatch& P = h->hp[p];
         const int ftx = P.prec == PREC_F32 ? Fused3<float>::TX : Fused3<double>::TX;

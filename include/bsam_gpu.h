@@ -77,13 +77,18 @@ int bsam_gpu_create(bsam_gpu** h, int device, const bsam_run_params* p);
  * them: every choice computes the same arithmetic in the same order.
  *   fuse_smoother  -1 automatic, 0 one launch per colour pass, 1 fused stage
  *                  (all 2*nu passes of LevelRelax in one launch) where the
- *                  level allows it
+ *                  level allows it: 3D levels.  2D levels at and below the
+ *                  root, of one patch and at most two sweeps, always run as
+ *                  such stages above the bottom chain, unless bottom_cells
+ *                  is -1
  *   fuse_min_n     smallest extent per dimension of a fused level
  *   chunk          planes (3D) / rows (2D) per streaming chunk, 0 = automatic
  *   bottom_cells   levels of at most this many cells run their whole part of
  *                  the V-cycle in one launch (a thread-block cluster, the
  *                  levels in its shared memory) as far as they fit there;
- *                  0 = default (as many levels as fit), -1 = never.  In the
+ *                  0 = default (those that cost less there: a whole problem
+ *                  that fits, else levels of at most 128^2 cells, 8192 in 3D),
+ *                  -1 = never, and every level one launch per pass.  In the
  *                  mixed form levels of at most bottom_cells are FP64; under
  *                  the default and with -1, levels of at most 4096 cells are
  *                  (the bits do not depend on which of them run in that launch)

@@ -1,0 +1,86 @@
+"""Whole smoothing stages of a wide 2D level with their transfers in one launch
+(k_stage2) against the same levels as one launch per pass (bottom_cells=-1),
+which the parity tests pin: every value the same bit for bit, at extents that
+are smaller than a tile, one tile, and not a multiple of either tile height or
+the tile width, each face rule, one or two sweeps, FP64 and mixed."""
+import ctypes
+
+import numpy as np
+import pytest
+
+import bsam_b200 as B
+from bsam_b200 import workloads as W
+
+pytestmark = pytest.mark.gpu
+
+FACES = {"neumann": [1, 1, 1, 1], "user": [10, 10, 10, 10], "periodic_x": [2, 2, 10, 10],
+         "periodic_y": [1, 1, 2, 2], "periodic": [2, 2, 2, 2]}
+
+
+def problem(mx, faces, sweeps=2):
+    core = list(mx)  # a periodic dimension is even or 1 on every level
+    while all(n % 2 == 0 for n in core):
+        core = [n // 2 for n in core]
+    for d in range(2):
+        if FACES[faces][2 * d] == 2 and core[d] % 2 and core[d] > 1:
+            pytest.skip("not a periodic extent")
+    rng = np.random.default_rng(int(np.prod(mx)))
+    h = 1.0 / mx[0]
+    return W.Problem(ndims=2, mx=(mx[0], mx[1], 1), eps=0.02, dt=1e-4, nsteps=2,
+                     qerrortol=1e-12, maxvcycles=3, nsmoothingpasses=sweeps,
+                     mthbc=tuple(FACES[faces]) + (1, 1),
+                     xupper=(1.0, mx[1] * h, 1.0),
+                     c0=0.5 + 0.1 * rng.uniform(-1, 1, int(np.prod(mx))))
+
+
+def solve(prob, precision, bottom_cells):
+    with B.Solver(prob, precision=precision, bottom_cells=bottom_cells) as s:
+        steps = [s.step() for _ in range(prob.nsteps)]
+        return steps, s.trace(), s.get_q()
+
+
+def same(got, want):
+    assert got[0] == want[0]
+    assert np.array_equal(got[1], want[1])
+    assert np.array_equal(got[2], want[2])
+
+
+# A chain of 16 cells at most: every larger level runs its stages as tiles.
+@pytest.mark.parametrize("sweeps", [1, 2, 3])
+@pytest.mark.parametrize("faces", sorted(FACES))
+@pytest.mark.parametrize("mx", [(8, 8), (16, 4), (4, 32), (32, 8), (64, 16), (40, 24), (72, 136), (64, 72),
+                                (128, 8), (8, 256), (64, 128)])
+def test_small_levels(gpu_lib, mx, faces, sweeps):
+    prob = problem(mx, faces, sweeps)
+    same(solve(prob, B.PREC_FP64, 16), solve(prob, B.PREC_FP64, -1))
+
+
+@pytest.mark.parametrize("precision", [B.PREC_FP64, B.PREC_MIXED])
+@pytest.mark.parametrize("faces", ["user", "periodic_x", "periodic"])
+@pytest.mark.parametrize("mx", [(320, 200), (384, 416), (264, 776), (1032, 520), (512, 512)])
+def test_wide_levels(gpu_lib, mx, faces, precision):
+    prob = problem(mx, faces)
+    same(solve(prob, precision, 0), solve(prob, precision, -1))
+
+
+@pytest.mark.parametrize("faces", ["user", "periodic"])
+def test_first_sweep_reads_the_ghosts_as_given(gpu_lib, faces):
+    prob = problem((64, 48), faces)
+    q0 = prob.q0()
+    rng = np.random.default_rng(3)
+    ring = np.ones(q0.shape[:2], dtype=bool)
+    ring[1:-1, 1:-1] = False
+    q0[ring] += 0.01 * rng.standard_normal((int(ring.sum()), 2))
+    out = []
+    for cells in (-1, 16):
+        with B.Solver(prob, bottom_cells=cells) as s:
+            s.put_q(q0)  # and no SetGhost
+            L = B.lib()
+            nv, conv, res = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_double(0.0)
+            assert L.bsam_gpu_copy_q_to_qold(s.h) == 0
+            assert L.bsam_gpu_multigrid_iterations(s.h, ctypes.byref(nv), ctypes.byref(res),
+                                                   ctypes.byref(conv)) == 0
+            out.append((nv.value, res.value, s.trace(), s.get_q()))
+    assert out[0][:2] == out[1][:2]
+    assert np.array_equal(out[0][2], out[1][2])
+    assert np.array_equal(out[0][3], out[1][3])
