@@ -422,13 +422,12 @@ template <int D>
 __device__ __forceinline__ void filldown_item(const DevPatch* __restrict__ PT, const Item it) {
   const DevPatch C = PT[it.patch];
   const DevPatch P = PT[C.parent];
-  const int jc = it.ty * TILE_Y + threadIdx.y + 1;
-  const int kc = D == 3 ? it.tz + 1 : 0;
+  const WorkPlace<D> w(it, C.cn[0]);
+  const int jc = w.j, kc = w.k;
   if (jc > C.cn[1]) return;
-  const int ic0 = (it.tx * 32 + threadIdx.x) * 2 + 1;
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int ic = ic0 + t;
+    const int ic = w.a0 + t * w.W;
     if (ic > C.cn[0]) break;
     const int i = 2 * ic, j = 2 * jc, k = 2 * kc;
     double val[2];

@@ -79,7 +79,7 @@ struct BatchCtl {
 };
 
 template <class T, int D>
-__global__ void __launch_bounds__(BLOCK_THREADS)
+__global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_relax(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
              const int* __restrict__ count, int color, TileRuns R) {
   const int n = *count;
@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS)
 // Transfers between a depth-d record (value type TC) and its parent, whose
 // type is the record's pprec.
 template <class TC, int D>
-__global__ void __launch_bounds__(BLOCK_THREADS)
+__global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_restrict(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                 const int* __restrict__ count, TileRuns R) {
   const int n = *count;
@@ -100,10 +100,9 @@ __global__ void __launch_bounds__(BLOCK_THREADS)
   }
 }
 
-// Eight CTAs per SM (a 64-register cap): 1.4 % faster per batch solve than
-// the compiler's 80 registers at six, despite a few spilled values.
+// As many CTAs per SM as hold a thread's block of children in registers.
 template <class TC, int D>
-__global__ void __launch_bounds__(BLOCK_THREADS, 8)
+__global__ void __launch_bounds__(BLOCK_THREADS, (sizeof(TC) == 4 ? 2 : 1) + (D == 2 ? 4 : 2))
     kb_coarse_load(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                    const int* __restrict__ count, TileRuns R) {
   const int n = *count;
@@ -115,7 +114,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
 }
 
 template <class TC, int D>
-__global__ void __launch_bounds__(BLOCK_THREADS)
+__global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_correct(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                const int* __restrict__ count, TileRuns R) {
   const int n = *count;
@@ -123,74 +122,6 @@ __global__ void __launch_bounds__(BLOCK_THREADS)
     const Item it = items[b];
     if (PT[it.patch].pprec == PREC_F32) correct_item<TC, float, D>(PT, it);
     else correct_item<TC, double, D>(PT, it);
-  }
-}
-
-// CorrectFine in 2D by 2 x 2 blocks of fine cells: the fine cells 2m, 2m+1
-// (x) and 2n, 2n+1 (y) read the same four parent corrections, formed once
-// here; each cell then takes correct_cell's bilinear expression on them, so
-// the values are correct_cell's bit for bit.  Block (m, n) for
-// m = 0..cn0, n = 0..cn1 covers fine cells 1..n0 x 1..n1 exactly once.
-template <class TC, class TP>
-__device__ __forceinline__ void correct_block2(const DevPatch& C, const DevPatch& P, int m,
-                                               int n) {
-  TC* q0 = fld<TC>(mid_state(C)[0]);
-  TC* q1 = fld<TC>(mid_state(C)[1]);
-  TP e[2][2][2];  // [component][m + a][n + b]
-#pragma unroll
-  for (int v = 0; v < 2; ++v) {
-    const TP* pq = fld<TP>(P.q[v]);
-    const TP* ps = fld<TP>(P.qs[v]);
-#pragma unroll
-    for (int a = 0; a < 2; ++a)
-#pragma unroll
-      for (int bb = 0; bb < 2; ++bb) {
-        const int64_t x = cidx(P, C.off[0] + m + a, C.off[1] + n + bb, 0);
-        e[v][a][bb] = pq[x] - ps[x];
-      }
-  }
-#pragma unroll
-  for (int dy = 0; dy < 2; ++dy) {
-    const int J = 2 * n + dy;
-    if (J < 1 || J > C.n[1]) continue;
-    const bool ey = dy == 0;
-#pragma unroll
-    for (int dx = 0; dx < 2; ++dx) {
-      const int I = 2 * m + dx;
-      if (I < 1 || I > C.n[0]) continue;
-      const bool ex = dx == 0;
-      TP corr[2];
-#pragma unroll
-      for (int v = 0; v < 2; ++v) {
-        const TP b0 = lin_x<TP>(ex, e[v][0][0], e[v][1][0]);
-        const TP b1 = lin_x<TP>(ex, e[v][0][1], e[v][1][1]);
-        corr[v] = lin_x<TP>(ey, b0, b1) / TP(16);
-      }
-      const int64_t c = cidx(C, I, J, 0);
-      const TC a0 = q0[c] + TC(corr[0]);
-      const TC a1 = q1[c] + TC(corr[1]);
-      q0[c] = a0;
-      q1[c] = a1;
-      if (C.wt && near_boundary(C, I, J, 0, 2)) write_through<TC, 2>(C, q0, q1, I, J, 0, a0, a1);
-    }
-  }
-}
-
-// Items: tiles of 32 x TILE_Y blocks (m, n) of a record (list L_CORR).
-template <class TC>
-__global__ void __launch_bounds__(BLOCK_THREADS, BATCH_LATENCY_MIN_BLOCKS)
-    kb_correct2(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
-                const int* __restrict__ count, TileRuns R) {
-  const int n = *count;
-  for (int b = R.first(); b < n; b = R.next(b)) {
-    const Item it = items[b];
-    const DevPatch C = PT[it.patch];
-    if (!C.active) continue;
-    const int m = it.tx * 32 + threadIdx.x, nn = it.ty * TILE_Y + threadIdx.y;
-    if (m > C.cn[0] || nn > C.cn[1]) continue;
-    const DevPatch P = PT[C.parent];
-    if (C.pprec == PREC_F32) correct_block2<TC, float>(C, P, m, nn);
-    else correct_block2<TC, double>(C, P, m, nn);
   }
 }
 
@@ -260,17 +191,13 @@ __global__ void __launch_bounds__(BLOCK_THREADS, BATCH_LATENCY_MIN_BLOCKS)
 }
 
 template <int D>
-__global__ void __launch_bounds__(BLOCK_THREADS, BATCH_LATENCY_MIN_BLOCKS)
+__global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_update(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
               const int* __restrict__ count, TileRuns R) {
   const int n = *count;
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];
-    const DevPatch M = PT[it.patch];
-    if (!M.active) continue;
-    const DevPatch& W = PT[M.twin];
-    if (W.fused) continue;  // updated by its post-smoothing stage (kb_smooth2, upd)
-    if (W.prec == PREC_F32) update_item<float, D>(PT, it);
+    if (PT[it.patch].prec == PREC_F32) update_item<float, D>(PT, it);
     else update_item<double, D>(PT, it);
   }
 }
@@ -295,31 +222,6 @@ __global__ void __launch_bounds__(D == 2 ? 128 : 256, D == 2 ? 8 : 4)
     if (!PT[it.patch].active) continue;  // uniform per CTA
     if (D == 2) ghost2_patch(PT, it.patch, cps, make_int2(it.tx, it.ty), ipass);
     else ghost3_patch(PT, it.patch, cps, make_int2(it.tx, it.ty), ipass);
-  }
-}
-
-// One colour pass (RelaxGrid2D + write-through) over tiles shaped to narrow
-// patches: refined patches are 8-64 cells wide, so the 64-column tiles of
-// kb_relax leave most lanes idle.  items[b] = {record, tile x, tile y, W}:
-// W lanes per row (8, 16 or 32) each take a column pair, 128 / W rows per
-// tile; the cell of the pass's colour in each pair is updated as relax_item
-// updates it, so the pass is the same whatever the tile shape.
-__global__ void __launch_bounds__(BLOCK_THREADS)
-    kb_relax_narrow2(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
-                     const int* __restrict__ count, int color, TileRuns R) {
-  const int n = *count;
-  const int t = threadIdx.x + blockDim.x * threadIdx.y;
-  for (int b = R.first(); b < n; b = R.next(b)) {
-    const Item it = items[b];
-    const DevPatch P = PT[it.patch];
-    if (!P.active) continue;  // uniform per CTA
-    const int W = it.tz;
-    const int j = it.ty * (BLOCK_THREADS / W) + t / W + 1;
-    if (j > P.n[1]) continue;
-    const int i0 = (it.tx * W + t % W) * 2 + 1;
-    const int i = i0 + ((i0 + j + color) & 1);
-    if (i > P.n[0]) continue;
-    relax_cell<double, 2>(P, i, j, 0);
   }
 }
 

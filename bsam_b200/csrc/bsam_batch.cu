@@ -60,31 +60,29 @@ constexpr int kDefaultTileChunk = 2;
 constexpr int kDefaultFusedChunk = 1;
 // Runs of the staged defect, in units of tile_chunk.
 constexpr int kDefectRunFactor = 4;
-// Lists: master tiles; bottom-chain tops; per top depth d: tiles of every
-// record (correction), footprint tiles (restriction / coarse load), tiles of
-// records smoothed per colour pass, fused-stage tiles; master tiles whose FP64
-// update is not done by their post-smoothing stage (mixed form, finest
-// working level not fused).
+// Lists: master tiles (sums); bottom-chain tops; per top depth d: footprint
+// tiles (coarse load), tiles of records smoothed per colour pass, fused-stage
+// tiles, blocks of records corrected and footprint tiles of records restricted
+// by a kernel of their own (not by a fused stage); tiles of the finest working
+// records whose master is updated by kb_update (mixed form, not fused).
 enum {
   L_MASTER = 0,
   L_TOPS = 1,
-  L_FINE = 2,
-  L_COARSE = 2 + MAXD,
-  L_RELAX = 2 + 2 * MAXD,
-  L_FUSED = 2 + 3 * MAXD,
-  L_CORR = 2 + 4 * MAXD,  // 2D: tiles of 2 x 2 fine-cell blocks (kb_correct2)
+  L_COARSE = 2,
+  L_RELAX = 2 + MAXD,
+  L_FUSED = 2 + 2 * MAXD,
+  L_CORR = 2 + 3 * MAXD,
+  L_RESTR = 2 + 4 * MAXD,
   L_UPD = 2 + 5 * MAXD,
-  L_RESTR = 3 + 5 * MAXD,  // footprint tiles of records restricted by kb_restrict
-  NLIST = 3 + 6 * MAXD
+  NLIST = 3 + 5 * MAXD
 };
 
 // Lists of the refined hierarchies (SLOT_AMR), over the records of their own
 // table: finest-level tiles (ErrorAFAS), bottom-chain tops; per depth d (up
-// to MAXD, the depth below the last top one included): interior tiles
-// (colour passes, correction), footprint tiles (restriction, coarse load),
-// footprint tiles of refined records (FillDown), refined records with their
-// GhostOverlap transfers (SetGhost), rows of partly covered parents
-// (snapshot).
+// to MAXD, the depth below the last top one included): interior tiles (colour
+// passes), footprint tiles (restriction, coarse load), footprint tiles of
+// refined records (FillDown), refined records with their GhostOverlap transfers
+// (SetGhost), rows of partly covered parents (snapshot), blocks (correction).
 enum {
   A_MASTER = 0,
   A_TOPS = 1,
@@ -93,7 +91,7 @@ enum {
   A_FILL = 2 + 2 * (MAXD + 1),
   A_GHOST = 2 + 3 * (MAXD + 1),
   A_SNAP = 2 + 4 * (MAXD + 1),
-  A_RELAX = 2 + 5 * (MAXD + 1),  // 2D: colour-pass tiles shaped to the patch width
+  A_CORR = 2 + 5 * (MAXD + 1),
   ANLIST = 2 + 6 * (MAXD + 1)
 };
 
@@ -581,18 +579,17 @@ void append_items(bsam_batch* b, int s) {
   tiles_for(rec0 + S.master, S.recs[S.master].n, nd, b->lists[L_MASTER].h);
   C.ie = (int)b->lists[L_MASTER].h.size();
   if (b->mixed && !S.recs[1].fused)
-    tiles_for(rec0 + S.master, S.recs[S.master].n, nd, b->lists[L_UPD].h);
+    work_tiles(rec0 + 1, S.recs[1].n, nd, b->lists[L_UPD].h);
   b->lists[L_TOPS].h.push_back(Item{S.top, 0, 0, 0});
   const int first = b->mixed ? 1 : 0;  // record of depth 0
   for (int d = 0; d < S.ntop; ++d) {
     const int r = first + d;
     const DevPatch& P = S.recs[r];
-    tiles_for(rec0 + r, P.n, nd, b->lists[L_FINE + d].h);
-    tiles_for(rec0 + r, P.cn, nd, b->lists[L_COARSE + d].h);
+    work_tiles(rec0 + r, P.cn, nd, b->lists[L_COARSE + d].h);
     // A 2D fused record's restriction is done by its pre-smoothing stage.
-    if (!(nd == 2 && P.fused)) tiles_for(rec0 + r, P.cn, nd, b->lists[L_RESTR + d].h);
+    if (!(nd == 2 && P.fused)) work_tiles(rec0 + r, P.cn, nd, b->lists[L_RESTR + d].h);
     if (!P.fused) {
-      tiles_for(rec0 + r, P.n, nd, b->lists[L_RELAX + d].h);
+      work_tiles(rec0 + r, P.n, nd, b->lists[L_RELAX + d].h);
     } else {
       const int tx = P.prec == PREC_F32 ? Fused2<float>::TX : Fused2<double>::TX;
       const int ty = P.prec == PREC_F32 ? Fused2<float>::TY : Fused2<double>::TY;
@@ -600,12 +597,8 @@ void append_items(bsam_batch* b, int s) {
         for (int x = 0; x < (P.n[0] + tx - 1) / tx; ++x)
           b->lists[L_FUSED + d].h.push_back(Item{rec0 + r, x, y, 0});
     }
-    // blocks (m, n), m = 0..cn0, n = 0..cn1, 32 x TILE_Y per tile; a fused
-    // record's correction is applied by its post-smoothing stage instead.
-    if (nd == 2 && !P.fused)
-      for (int y = 0; y < (P.cn[1] + 1 + TILE_Y - 1) / TILE_Y; ++y)
-        for (int x = 0; x < (P.cn[0] + 1 + 31) / 32; ++x)
-          b->lists[L_CORR + d].h.push_back(Item{rec0 + r, x, y, 0});
+    // A fused record's correction is applied by its post-smoothing stage.
+    if (!P.fused) block_tiles(rec0 + r, P.cn, nd, b->lists[L_CORR + d].h);
   }
   b->cfg_dirty = true;
 }
@@ -706,19 +699,11 @@ void amr_append(bsam_batch* b, int s, bool active) {
       for (size_t k = 0; k < E.patches.size(); ++k) {
         const int p = E.patches[k];
         const DevPatch& P = V.recs[p];
-        tiles_for(r0 + p, P.n, nd, LA[A_FINE + d].h);
-        if (nd == 2) {
-          // W lanes per row: the narrowest of 8, 16, 32 whose 2W columns
-          // cover the patch (or 32).
-          const int W = P.n[0] <= 16 ? 8 : (P.n[0] <= 32 ? 16 : 32);
-          const int rows = BLOCK_THREADS / W;
-          for (int y = 0; y < (P.n[1] + rows - 1) / rows; ++y)
-            for (int x = 0; x < (P.n[0] + 2 * W - 1) / (2 * W); ++x)
-              LA[A_RELAX + d].h.push_back(Item{r0 + p, x, y, W});
-        }
-        tiles_for(r0 + p, P.cn, nd, LA[A_COARSE + d].h);
+        work_tiles(r0 + p, P.n, nd, LA[A_FINE + d].h);
+        work_tiles(r0 + p, P.cn, nd, LA[A_COARSE + d].h);
+        block_tiles(r0 + p, P.cn, nd, LA[A_CORR + d].h);
         if (E.amr) {
-          tiles_for(r0 + p, P.cn, nd, LA[A_FILL + d].h);
+          work_tiles(r0 + p, P.cn, nd, LA[A_FILL + d].h);
           const int2 rg = k < E.range.size() ? E.range[k] : make_int2(0, 0);
           LA[A_GHOST + d].h.push_back(Item{r0 + p, ob + rg.x, rg.y, 0});
         }
@@ -919,12 +904,8 @@ void tick_t(bsam_batch* b, cudaGraphConditionalHandle handle, int in_graph) {
     if (LA[A_FINE + d].cap == 0) return;
     for (int pass = 0; pass < nu; ++pass)
       for (int color = 0; color < 2; ++color) {
-        if (D == 2)
-          kb_relax_narrow2<<<agrid(A_RELAX + d), blk, 0, s>>>(apt, LA[A_RELAX + d].d,
-                                                              acnt + A_RELAX + d, color, R);
-        else
-          kb_relax<double, D><<<agrid(A_FINE + d), blk, 0, s>>>(apt, LA[A_FINE + d].d,
-                                                                acnt + A_FINE + d, color, R);
+        kb_relax<double, D><<<agrid(A_FINE + d), blk, 0, s>>>(apt, LA[A_FINE + d].d,
+                                                              acnt + A_FINE + d, color, R);
         ++n;
         aghost(d, color + 1);
       }
@@ -1042,29 +1023,19 @@ void tick_t(bsam_batch* b, cudaGraphConditionalHandle handle, int in_graph) {
     }
   }
   for (int d = b->cap_depth - 1; d >= 0; --d) {
-    if (D == 2) {
-      // Records with fused stages are corrected by their post-smoothing stage.
-      if (L[L_CORR + d].cap > 0) {
-        const int gk = grid_for(b, L_CORR + d);
-        if (b->mixed)
-          kb_correct2<float><<<gk, blk, 0, s>>>(pt, L[L_CORR + d].d, cnt + L_CORR + d, R);
-        else
-          kb_correct2<double><<<gk, blk, 0, s>>>(pt, L[L_CORR + d].d, cnt + L_CORR + d, R);
-      } else {
-        --n;
-      }
-    } else {
-      const int gf = grid_for(b, L_FINE + d);
+    // Records with fused stages are corrected by their post-smoothing stage.
+    if (L[L_CORR + d].cap > 0) {
+      const int gk = grid_for(b, L_CORR + d);
       if (b->mixed)
-        kb_correct<float, D><<<gf, blk, 0, s>>>(pt, L[L_FINE + d].d, cnt + L_FINE + d, R);
+        kb_correct<float, D><<<gk, blk, 0, s>>>(pt, L[L_CORR + d].d, cnt + L_CORR + d, R);
       else
-        kb_correct<double, D><<<gf, blk, 0, s>>>(pt, L[L_FINE + d].d, cnt + L_FINE + d, R);
+        kb_correct<double, D><<<gk, blk, 0, s>>>(pt, L[L_CORR + d].d, cnt + L_CORR + d, R);
+      ++n;
     }
-    ++n;
     if (LA[A_FINE + d].cap > 0) {
       // CorrectFine and SetGhost(level, 0) (afas:513-515).
-      kb_correct<double, D><<<agrid(A_FINE + d), blk, 0, s>>>(apt, LA[A_FINE + d].d,
-                                                              acnt + A_FINE + d, R);
+      kb_correct<double, D><<<agrid(A_CORR + d), blk, 0, s>>>(apt, LA[A_CORR + d].d,
+                                                              acnt + A_CORR + d, R);
       ++n;
       aghost(d, 0);
     }

@@ -63,7 +63,9 @@ struct LevelPlan {
   Item* d_fine = nullptr;    // tiles over each patch's interior
   int nfine = 0;
   Item* d_coarse = nullptr;  // tiles over each patch's footprint in its parent
+  Item* d_corr = nullptr;    // tiles over each patch's blocks for the correction
   int ncoarse = 0;
+  int ncorr = 0;
   Item* d_fused = nullptr;   // fused-stage tiles (tile x, tile y, z chunk)
   int nfused = 0;
   bool fused = false;
@@ -323,7 +325,7 @@ void launch_transfer_t(bsam_gpu* h, const LevelPlan& L, int what) {
   else if (what == 2)
     k_coarse_load<TC, TP, D><<<L.ncoarse, block_dim(), 0, h->stream>>>(h->d_patches, L.d_coarse);
   else
-    k_correct<TC, TP, D><<<L.nfine, block_dim(), 0, h->stream>>>(h->d_patches, L.d_fine);
+    k_correct<TC, TP, D><<<L.ncorr, block_dim(), 0, h->stream>>>(h->d_patches, L.d_corr);
 }
 
 // SetGhost(level, ipass) of a refined level (boundary.f90:58-89): coarse-fine
@@ -534,14 +536,15 @@ void launch_resid(bsam_gpu* h) {
 // Mixed form: q64 += q32 - fl32(q64) after the FP32 V-cycle.
 void launch_update(bsam_gpu* h) {
   const int nd = h->rp.ndims;
-  const bool f32 = plan(h, h->finestlevel).prec == PREC_F32;
+  const LevelPlan& L = plan(h, h->finestlevel);  // the twins' tiles
+  const bool f32 = L.prec == PREC_F32;
   const dim3 b = block_dim();
   if (nd == 2) {
-    if (f32) k_update<float, 2><<<h->nmaster, b, 0, h->stream>>>(h->d_patches, h->d_master);
-    else k_update<double, 2><<<h->nmaster, b, 0, h->stream>>>(h->d_patches, h->d_master);
+    if (f32) k_update<float, 2><<<L.nfine, b, 0, h->stream>>>(h->d_patches, L.d_fine);
+    else k_update<double, 2><<<L.nfine, b, 0, h->stream>>>(h->d_patches, L.d_fine);
   } else {
-    if (f32) k_update<float, 3><<<h->nmaster, b, 0, h->stream>>>(h->d_patches, h->d_master);
-    else k_update<double, 3><<<h->nmaster, b, 0, h->stream>>>(h->d_patches, h->d_master);
+    if (f32) k_update<float, 3><<<L.nfine, b, 0, h->stream>>>(h->d_patches, L.d_fine);
+    else k_update<double, 3><<<L.nfine, b, 0, h->stream>>>(h->d_patches, L.d_fine);
   }
   ++h->stats.launches;
 }
@@ -1307,7 +1310,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
   // Level precisions and work lists.
   std::vector<Item> all;
   const size_t nl = h->levels.size();
-  std::vector<std::pair<int, int>> spans_fine(nl), spans_coarse(nl), spans_fused(nl);
+  std::vector<std::pair<int, int>> spans_fine(nl), spans_coarse(nl), spans_corr(nl), spans_fused(nl);
   for (size_t li = 0; li < nl; ++li) {
     LevelPlan& L = h->levels[li];
     if (L.patches.empty()) return fail(h, BSAM_ERR_ARG, "a level between minlevel and finest is empty");
@@ -1315,12 +1318,16 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     for (int p : L.patches)
       if (h->hp[p].prec != L.prec) return fail(h, BSAM_ERR_ARG, "mixed precisions on one level");
     int s = (int)all.size();
-    for (int p : L.patches) tiles_for(p, h->hp[p].n, nd, all);
+    for (int p : L.patches) work_tiles(p, h->hp[p].n, nd, all);
     spans_fine[li] = {s, (int)all.size() - s};
     s = (int)all.size();
     for (int p : L.patches)
-      if (h->hp[p].parent >= 0) tiles_for(p, h->hp[p].cn, nd, all);
+      if (h->hp[p].parent >= 0) work_tiles(p, h->hp[p].cn, nd, all);
     spans_coarse[li] = {s, (int)all.size() - s};
+    s = (int)all.size();
+    for (int p : L.patches)
+      if (h->hp[p].parent >= 0) block_tiles(p, h->hp[p].cn, nd, all);
+    spans_corr[li] = {s, (int)all.size() - s};
     // A level runs fused stages only when every patch on it does.
     L.fused = true;
     for (int p : L.patches) L.fused = L.fused && h->hp[p].fused;
@@ -1440,6 +1447,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     L.novl = span_ovl[li].second;
     L.nfine = spans_fine[li].second;
     L.ncoarse = spans_coarse[li].second;
+    L.ncorr = spans_corr[li].second;
     L.nfused = spans_fused[li].second;
     h->max_items = std::max(h->max_items, L.nfine);
   }
@@ -1528,6 +1536,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
                           : reinterpret_cast<int2*>(base + o_ovl_rng) + span_plist[li].first;
       L.d_fine = h->d_items + spans_fine[li].first;
       L.d_coarse = h->d_items + spans_coarse[li].first;
+      L.d_corr = h->d_items + spans_corr[li].first;
       L.d_fused = h->d_items + spans_fused[li].first;
     }
     h->d_master = h->d_items + s_master;

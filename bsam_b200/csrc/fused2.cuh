@@ -360,7 +360,7 @@ __device__ __forceinline__ void smooth_band(T* s0, T* s1, const T* sf0, const T*
 // CorrectFine (afas:842-963) of the cells of a shared tile: every cell of the
 // tile inside the patch's interior takes the bilinear prolongation of the
 // parent's q - qs (the change of the coarse solution), the expression of
-// correct_block2, so the tile holds what kb_correct2 would have written.
+// correct_block, so the tile holds what kb_correct would have written.
 template <class T, class TP>
 __device__ __forceinline__ void correct_tile2(const DevPatch& C, const DevPatch& R, T* s0, T* s1,
                                               int gx0, int gy0) {
@@ -462,7 +462,7 @@ __device__ __forceinline__ void restrict_tile2(const DevPatch& C, const DevPatch
 // which nothing else in the launch reads.
 // corr (post-smoothing): the coarse-grid correction is applied to the tile
 // after it lands (correct_tile2, then the physical face ghosts the passes
-// read), instead of by a kb_correct2 launch before the stage.
+// read), instead of by a kb_correct launch before the stage.
 // restr (pre-smoothing): the tile's coarse cells are restricted into the
 // parent from shared memory (restrict_tile2), instead of by a kb_restrict
 // launch after the stage.

@@ -16,6 +16,8 @@
 // dimensions ends up as the map of each face in S (ascending dimension)
 // applied to the interior cell reflected across all of S.
 #pragma once
+#include <vector>
+
 #include <algorithm>
 
 #include "bsam_types.h"
@@ -49,6 +51,49 @@ __device__ __forceinline__ void* const* mid_state(const DevPatch& P) {
 __device__ __forceinline__ int64_t cidx(const DevPatch& P, int i, int j, int k) {
   return (int64_t)i + (int64_t)j * P.sy + (int64_t)k * P.sz;
 }
+
+// Two neighbouring cells of a row, the first of odd index: rows start so that
+// cell 1 is 128-byte aligned, so the pair is one aligned load.
+template <class T> struct PairOf;
+template <> struct PairOf<float> { using V = float2; };
+template <> struct PairOf<double> { using V = double2; };
+template <class T>
+__device__ __forceinline__ typename PairOf<T>::V load_pair(const T* p) {
+  return *reinterpret_cast<const typename PairOf<T>::V*>(p);
+}
+
+// ---- work tiles --------------------------------------------------------------
+//
+// Tiles of the kernels whose result does not depend on which thread takes which
+// cell (all but the sums, whose tiles are TILE_X x TILE_Y): W lanes a row, two
+// cells a lane, BLOCK_THREADS / W rows of one plane.  W is the least power of
+// two that covers a row, up to a warp: on rows of 24 cells the fixed 32 lanes
+// left 20 of them idle.
+__host__ __device__ inline int work_lanes(int n0) {
+  return n0 <= 8 ? 4 : n0 <= 16 ? 8 : n0 <= 32 ? 16 : 32;
+}
+
+inline void work_tiles(int patch, const int* n, int nd, std::vector<Item>& out) {
+  const int W = work_lanes(n[0]), rows = BLOCK_THREADS / W;
+  for (int z = 0; z < (nd == 3 ? n[2] : 1); ++z)
+    for (int y = 0; y < (n[1] + rows - 1) / rows; ++y)
+      for (int x = 0; x < (n[0] + 2 * W - 1) / (2 * W); ++x) out.push_back(Item{patch, x, y, z});
+}
+
+// A thread's place in a work tile: its pair of cells starts at i0; as two
+// strided cells it takes a0 and a0 + W.
+template <int D>
+struct WorkPlace {
+  int W, i0, a0, j, k;
+  __device__ __forceinline__ WorkPlace(const Item& it, int n0) {
+    W = work_lanes(n0);
+    const int t = threadIdx.x + 32 * threadIdx.y, lane = t & (W - 1);
+    j = it.ty * (BLOCK_THREADS / W) + t / W + 1;
+    k = D == 3 ? it.tz + 1 : 0;
+    i0 = 2 * (it.tx * W + lane) + 1;
+    a0 = 2 * it.tx * W + lane + 1;
+  }
+};
 
 template <class T> __device__ __forceinline__ T bc_map(int code, T v) {
   return code == BC_REFLECT ? T(2) - v : (code == BC_NEGATE ? -v : v);
@@ -175,6 +220,16 @@ __device__ __forceinline__ void operator_at(const DevPatch& P, const Problem::St
     Problem::OperatorCell<T, D>(s, T(P.tmp1), T(P.tmp2), T(P.alpha), o0, o1);
 }
 
+// The same with the base state's value given (correction form only).
+template <class T, int D>
+__device__ __forceinline__ void operator_with(const DevPatch& P, const Problem::Stencil<T, D>& s,
+                                              T base, T& o0, T& o1) {
+  if (P.delta)
+    Problem::OperatorCell<T, D, true>(s, T(P.tmp1), T(P.tmp2), T(P.alpha), o0, o1, base);
+  else
+    Problem::OperatorCell<T, D>(s, T(P.tmp1), T(P.tmp2), T(P.alpha), o0, o1);
+}
+
 // Residual rf = f - Operator(q) at one cell (afas:799-840).
 template <class T, int D>
 __device__ __forceinline__ void residual_cell(const DevPatch& P, const T* q0, const T* q1,
@@ -198,21 +253,20 @@ __device__ __forceinline__ void residual_cell(const DevPatch& P, const T* q0, co
 template <class TC, class TP, int D>
 __device__ __forceinline__ void restrict_cell(const DevPatch& C, const DevPatch& P, int ic, int jc,
                                               int kc) {
-  const int i = 2 * ic, j = 2 * jc, k = 2 * kc;
-  TP val[2];
+  // The block's cells, row by row from the high end, high cell first: the
+  // order of the sum.
+  const int64_t c0 = cidx(C, 2 * ic - 1, 2 * jc - 1, D == 3 ? 2 * kc - 1 : 0);
+  auto average = [&](const TC* a) {
+    TC s = TC(0);
 #pragma unroll
-  for (int v = 0; v < 2; ++v) {
-    const TC* a = fld<TC>(mid_state(C)[v]);
-    if (D == 2) {
-      val[v] = TP(TC(0.25) * (a[cidx(C, i, j, 0)] + a[cidx(C, i - 1, j, 0)] +
-                              a[cidx(C, i, j - 1, 0)] + a[cidx(C, i - 1, j - 1, 0)]));
-    } else {
-      val[v] = TP(TC(0.125) * (a[cidx(C, i, j, k)] + a[cidx(C, i - 1, j, k)] +
-                               a[cidx(C, i, j - 1, k)] + a[cidx(C, i - 1, j - 1, k)] +
-                               a[cidx(C, i, j, k - 1)] + a[cidx(C, i - 1, j, k - 1)] +
-                               a[cidx(C, i, j - 1, k - 1)] + a[cidx(C, i - 1, j - 1, k - 1)]));
+    for (int r = (D == 3 ? 3 : 1); r >= 0; --r) {
+      const auto v = load_pair<TC>(a + c0 + (r & 1) * C.sy + (r >> 1) * C.sz);
+      s = r == (D == 3 ? 3 : 1) ? v.y : s + v.y;
+      s = s + v.x;
     }
-  }
+    return TP((D == 3 ? TC(0.125) : TC(0.25)) * s);
+  };
+  const TP val[2] = {average(fld<TC>(mid_state(C)[0])), average(fld<TC>(mid_state(C)[1]))};
   const int pi = C.off[0] + ic, pj = C.off[1] + jc, pk = (D == 3) ? C.off[2] + kc : 0;
   const int64_t pc = cidx(P, pi, pj, pk);
   TP* pq0 = fld<TP>(P.q[0]);
@@ -229,43 +283,83 @@ __device__ __forceinline__ void restrict_cell(const DevPatch& C, const DevPatch&
   }
   if (P.delta) {
     // Correction form: the coarse base is the restriction of the fine base.
-    const TC* b = fld<TC>(C.bs);
-    if (D == 2)
-      fld<TP>(P.bs)[pc] = TP(TC(0.25) * (b[cidx(C, i, j, 0)] + b[cidx(C, i - 1, j, 0)] +
-                                         b[cidx(C, i, j - 1, 0)] + b[cidx(C, i - 1, j - 1, 0)]));
-    else
-      fld<TP>(P.bs)[pc] =
-          TP(TC(0.125) * (b[cidx(C, i, j, k)] + b[cidx(C, i - 1, j, k)] + b[cidx(C, i, j - 1, k)] +
-                          b[cidx(C, i - 1, j - 1, k)] + b[cidx(C, i, j, k - 1)] +
-                          b[cidx(C, i - 1, j, k - 1)] + b[cidx(C, i, j - 1, k - 1)] +
-                          b[cidx(C, i - 1, j - 1, k - 1)]));
+    fld<TP>(P.bs)[pc] = average(fld<TC>(C.bs));
   }
+}
+
+// The 2^D block of fine cells whose low corner is element c, with its face
+// neighbours: a[z][y][x], the block at indices 1 and 2 (2D: z = 0).  The rows
+// through the block come as aligned pairs, and each value is loaded once.
+template <class T, int D>
+__device__ __forceinline__ void load_block(const DevPatch& C, const T* __restrict__ q, int64_t c,
+                                           T (&a)[D == 3 ? 4 : 1][4][4]) {
+#pragma unroll
+  for (int z = 0; z < (D == 3 ? 4 : 1); ++z)
+#pragma unroll
+    for (int y = 0; y < 4; ++y) {
+      const bool zin = D == 2 || z == 1 || z == 2, yin = y == 1 || y == 2;
+      if (!zin && !yin) continue;
+      const T* p = q + c + (y - 1) * C.sy + (D == 3 ? (z - 1) * C.sz : 0);
+      const auto v = load_pair<T>(p);
+      a[z][y][1] = v.x;
+      a[z][y][2] = v.y;
+      if (zin && yin) {
+        a[z][y][0] = p[-1];
+        a[z][y][3] = p[2];
+      }
+    }
 }
 
 // CoarseLoadingFunction (afas:646-714) at one coarse cell:
 //   parent%f(mb) = Restriction(f - Operator(q)) + Operator(qc, h = parent%dx)
+// A thread holds its block of children with the neighbours in registers
+// (load_block).  Loaded cell by cell, with every second element of a row per
+// warp and 13 (2D) or 17 loads a child, the pass ran at 78 % of L1's rate and a
+// third of the memory's.  From a 128^3 FP64 level 41 -> 35 us, all levels of 24
+// problems of 32^3 and 64^3 (FP32) 130 -> 77, of 512 of 64^2 to 256^2 190 -> 175,
+// of 96 in FP64 100 -> 66; now the latency of the loads bounds it.
 template <class TC, class TP, int D>
 __device__ __forceinline__ void coarse_load_cell(const DevPatch& C, const DevPatch& P, int ic,
                                                  int jc, int kc) {
-  const TC* q0 = fld<TC>(mid_state(C)[0]);
-  const TC* q1 = fld<TC>(mid_state(C)[1]);
-  const TC* f0 = fld<TC>(C.f[0]);
-  const TC* f1 = fld<TC>(C.f[1]);
-  const int i = 2 * ic, j = 2 * jc, k = 2 * kc;
-  // Restriction of rf: children in the reference's summation order.
-  const int nch = (D == 2) ? 4 : 8;
+  const int64_t c0 = cidx(C, 2 * ic - 1, 2 * jc - 1, D == 3 ? 2 * kc - 1 : 0);
+  TC a[2][D == 3 ? 4 : 1][4][4];
+  load_block<TC, D>(C, fld<TC>(mid_state(C)[0]), c0, a[0]);
+  load_block<TC, D>(C, fld<TC>(mid_state(C)[1]), c0, a[1]);
+  // Restriction of rf: children in the reference's summation order, from the
+  // high end of each dimension.
   TC s0 = TC(0), s1 = TC(0);
 #pragma unroll
-  for (int ch = 0; ch < nch; ++ch) {
-    const int ii = i - (ch & 1), jj = j - ((ch >> 1) & 1), kk = (D == 3) ? k - (ch >> 2) : 0;
-    TC r0, r1;
-    residual_cell<TC, D>(C, q0, q1, f0, f1, cidx(C, ii, jj, kk), r0, r1);
-    if (ch == 0) {
-      s0 = r0;
-      s1 = r1;
-    } else {
-      s0 = s0 + r0;
-      s1 = s1 + r1;
+  for (int r = (D == 3 ? 3 : 1); r >= 0; --r) {
+    const int y = 1 + (r & 1), z = D == 3 ? 1 + (r >> 1) : 0;
+    const int64_t c = c0 + (r & 1) * C.sy + (r >> 1) * C.sz;
+    const auto f0 = load_pair<TC>(fld<TC>(C.f[0]) + c), f1 = load_pair<TC>(fld<TC>(C.f[1]) + c);
+    typename PairOf<TC>::V base{};
+    if (C.delta) base = load_pair<TC>(fld<TC>(C.bs) + c);
+#pragma unroll
+    for (int x = 2; x >= 1; --x) {
+      Problem::Stencil<TC, D> s;
+      s.pc = a[0][z][y][x];
+      s.mc = a[1][z][y][x];
+      s.pm[0] = a[0][z][y][x - 1];
+      s.pp[0] = a[0][z][y][x + 1];
+      s.mm[0] = a[1][z][y][x - 1];
+      s.mp[0] = a[1][z][y][x + 1];
+      s.pm[1] = a[0][z][y - 1][x];
+      s.pp[1] = a[0][z][y + 1][x];
+      s.mm[1] = a[1][z][y - 1][x];
+      s.mp[1] = a[1][z][y + 1][x];
+      if (D == 3) {
+        s.pm[D - 1] = a[0][D == 3 ? z - 1 : 0][y][x];
+        s.pp[D - 1] = a[0][D == 3 ? z + 1 : 0][y][x];
+        s.mm[D - 1] = a[1][D == 3 ? z - 1 : 0][y][x];
+        s.mp[D - 1] = a[1][D == 3 ? z + 1 : 0][y][x];
+      }
+      TC o0, o1;
+      operator_with<TC, D>(C, s, x == 2 ? base.y : base.x, o0, o1);
+      const TC r0 = (x == 2 ? f0.y : f0.x) - o0, r1 = (x == 2 ? f1.y : f1.x) - o1;
+      const bool first = x == 2 && r == (D == 3 ? 3 : 1);
+      s0 = first ? r0 : s0 + r0;
+      s1 = first ? r1 : s1 + r1;
     }
   }
   const TC w = (D == 2) ? TC(0.25) : TC(0.125);
@@ -333,6 +427,74 @@ __device__ __forceinline__ void correct_cell(const DevPatch& C, const DevPatch& 
   if (C.wt && near_boundary(C, I, J, K, D)) write_through<TC, D>(C, q0, q1, I, J, K, a0, a1);
 }
 
+// CorrectFine by 2^D blocks of fine cells: the fine cells 2m, 2m+1 of each
+// dimension read the same 2^D parent corrections, formed once here; each cell
+// then takes correct_cell's expression on them, so the values are
+// correct_cell's bit for bit.  Block (m, n, p) from 0 to cn of each dimension
+// covers the fine cells 1 to n exactly once.  Cell by cell a fine cell took 16
+// (2D) or 32 parent loads: 128^3 FP64 46 us, now 28; three levels of 24 problems
+// of 32^3 and 64^3 130 and 101 us.
+template <class TC, class TP, int D>
+__device__ __forceinline__ void correct_block(const DevPatch& C, const DevPatch& P, int m, int n,
+                                              int p) {
+  TC* q0 = fld<TC>(mid_state(C)[0]);
+  TC* q1 = fld<TC>(mid_state(C)[1]);
+  constexpr int NZ = D == 3 ? 2 : 1;
+  TP e[2][NZ][2][2];  // [component][p + c][n + b][m + a]
+  const int64_t x0 = cidx(P, C.off[0] + m, C.off[1] + n, D == 3 ? C.off[2] + p : 0);
+#pragma unroll
+  for (int v = 0; v < 2; ++v) {
+    const TP* pq = fld<TP>(P.q[v]) + x0;
+    const TP* ps = fld<TP>(P.qs[v]) + x0;
+#pragma unroll
+    for (int c = 0; c < NZ; ++c)
+#pragma unroll
+      for (int b = 0; b < 2; ++b)
+#pragma unroll
+        for (int a = 0; a < 2; ++a) {
+          const int64_t x = a + b * P.sy + c * P.sz;
+          e[v][c][b][a] = pq[x] - ps[x];
+        }
+  }
+#pragma unroll 1
+  for (int r = 0; r < 2 * NZ; ++r) {
+    const int dy = r & 1, dz = r >> 1;
+    const int J = 2 * n + dy, K = D == 3 ? 2 * p + dz : 0;
+    if (J < 1 || J > C.n[1] || (D == 3 && (K < 1 || K > C.n[2]))) continue;
+    // lin_x with the choice at run time; its two terms commute.
+    auto lin = [](bool even, TP a, TP b) { return TP(3) * (even ? a : b) + (even ? b : a); };
+#pragma unroll
+    for (int dx = 0; dx < 2; ++dx) {
+      const int I = 2 * m + dx;
+      if (I < 1 || I > C.n[0]) continue;
+      TP corr[2];
+#pragma unroll
+      for (int v = 0; v < 2; ++v) {
+        TP cz[NZ];
+#pragma unroll
+        for (int c = 0; c < NZ; ++c)
+          cz[c] = lin(dy == 0, lin_x<TP>(dx == 0, e[v][c][0][0], e[v][c][0][1]),
+                      lin_x<TP>(dx == 0, e[v][c][1][0], e[v][c][1][1]));
+        corr[v] = D == 3 ? lin(dz == 0, cz[0], cz[NZ - 1]) / TP(64) : cz[0] / TP(16);
+      }
+      const int64_t c = cidx(C, I, J, K);
+      const TC a0 = q0[c] + TC(corr[0]);
+      const TC a1 = q1[c] + TC(corr[1]);
+      q0[c] = a0;
+      q1[c] = a1;
+      if (C.wt && near_boundary(C, I, J, K, D)) write_through<TC, D>(C, q0, q1, I, J, K, a0, a1);
+    }
+  }
+}
+
+// Tiles of BLOCK_THREADS consecutive blocks of a patch, x fastest.
+inline void block_tiles(int patch, const int* cn, int nd, std::vector<Item>& out) {
+  int64_t blocks = nd == 3 ? cn[2] + 1 : 1;
+  blocks *= (int64_t)(cn[0] + 1) * (cn[1] + 1);
+  for (int64_t b = 0; b < blocks; b += BLOCK_THREADS)
+    out.push_back(Item{patch, (int)(b / BLOCK_THREADS), 0, 0});
+}
+
 // ---- reductions --------------------------------------------------------------
 
 // Deterministic block sum of a double (fixed shuffle tree + fixed smem
@@ -398,13 +560,11 @@ __device__ __forceinline__ void relax_item(const DevPatch* __restrict__ PT, cons
                                            int color) {
   const DevPatch P = PT[it.patch];  // by value: fields stay in registers
   if (!P.active) return;
-  const int j = it.ty * TILE_Y + threadIdx.y + 1;
-  const int k = (D == 3) ? it.tz + 1 : 0;
-  if (j > P.n[1]) return;
-  const int i0 = (it.tx * 32 + threadIdx.x) * 2 + 1;
-  const int i = i0 + ((i0 + j + k + color) & 1);
+  const WorkPlace<D> w(it, P.n[0]);
+  if (w.j > P.n[1]) return;
+  const int i = w.i0 + ((w.i0 + w.j + w.k + color) & 1);
   if (i > P.n[0]) return;
-  relax_cell<T, D>(P, i, j, k);
+  relax_cell<T, D>(P, i, w.j, w.k);
 }
 
 // Sum of rf^2 over this thread's cells of a tile (ErrorAFAS's SquareSum).
@@ -437,15 +597,13 @@ __device__ __forceinline__ void restrict_item(const DevPatch* __restrict__ PT, c
   const DevPatch C = PT[it.patch];
   if (!C.active) return;
   const DevPatch P = PT[C.parent];
-  const int jc = it.ty * TILE_Y + threadIdx.y + 1;
-  const int kc = (D == 3) ? it.tz + 1 : 0;
-  if (jc > C.cn[1]) return;
-  const int ic0 = (it.tx * 32 + threadIdx.x) * 2 + 1;
+  const WorkPlace<D> w(it, C.cn[0]);
+  if (w.j > C.cn[1]) return;
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int ic = ic0 + t;
+    const int ic = w.a0 + t * w.W;
     if (ic > C.cn[0]) break;
-    restrict_cell<TC, TP, D>(C, P, ic, jc, kc);
+    restrict_cell<TC, TP, D>(C, P, ic, w.j, w.k);
   }
 }
 
@@ -454,15 +612,13 @@ __device__ __forceinline__ void coarse_load_item(const DevPatch* __restrict__ PT
   const DevPatch C = PT[it.patch];
   if (!C.active) return;
   const DevPatch P = PT[C.parent];
-  const int jc = it.ty * TILE_Y + threadIdx.y + 1;
-  const int kc = (D == 3) ? it.tz + 1 : 0;
-  if (jc > C.cn[1]) return;
-  const int ic0 = (it.tx * 32 + threadIdx.x) * 2 + 1;
-#pragma unroll
+  const WorkPlace<D> w(it, C.cn[0]);
+  if (w.j > C.cn[1]) return;
+#pragma unroll 1
   for (int t = 0; t < 2; ++t) {
-    const int ic = ic0 + t;
+    const int ic = w.a0 + t * w.W;
     if (ic > C.cn[0]) break;
-    coarse_load_cell<TC, TP, D>(C, P, ic, jc, kc);
+    coarse_load_cell<TC, TP, D>(C, P, ic, w.j, w.k);
   }
 }
 
@@ -471,16 +627,12 @@ __device__ __forceinline__ void correct_item(const DevPatch* __restrict__ PT, co
   const DevPatch C = PT[it.patch];
   if (!C.active) return;
   const DevPatch P = PT[C.parent];
-  const int J = it.ty * TILE_Y + threadIdx.y + 1;
-  const int K = (D == 3) ? it.tz + 1 : 0;
-  if (J > C.n[1]) return;
-  const int I0 = (it.tx * 32 + threadIdx.x) * 2 + 1;
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
-    const int I = I0 + t;
-    if (I > C.n[0]) break;
-    correct_cell<TC, TP, D>(C, P, I, J, K);
-  }
+  int u = it.tx * BLOCK_THREADS + threadIdx.x + 32 * threadIdx.y;
+  const int m = u % (C.cn[0] + 1);
+  u /= C.cn[0] + 1;
+  const int n = D == 3 ? u % (C.cn[1] + 1) : u, p = D == 3 ? u / (C.cn[1] + 1) : 0;
+  if (D == 3 ? p > C.cn[2] : n > C.cn[1]) return;
+  correct_block<TC, TP, D>(C, P, m, n, p);
 }
 
 // GetSourceFunction + UpdateSourceFunction on one level (afas:312-367,

@@ -64,30 +64,29 @@ __device__ __forceinline__ double defect_item(const DevPatch* __restrict__ PT, c
   return acc;
 }
 
-// q64 += e on the interior of one master tile; ghosts by write-through.
+// q64 += e on one work tile of a twin; ghosts by write-through.
 template <class TW, int D>
 __device__ __forceinline__ void update_item(const DevPatch* __restrict__ PT, const Item it) {
-  const DevPatch M = PT[it.patch];
+  const DevPatch W = PT[it.patch];
+  const DevPatch M = PT[W.master];
   if (!M.active) return;
-  const DevPatch W = PT[M.twin];
-  const int j = it.ty * TILE_Y + threadIdx.y + 1;
-  const int k = (D == 3) ? it.tz + 1 : 0;
-  if (j > M.n[1]) return;
-  const int i0 = (it.tx * 32 + threadIdx.x) * 2 + 1;
+  const WorkPlace<D> w(it, M.n[0]);
+  if (w.j > M.n[1]) return;
   double* q0 = fld<double>(M.q[0]);
   double* q1 = fld<double>(M.q[1]);
   const TW* e0 = fld<TW>(W.q[0]);
   const TW* e1 = fld<TW>(W.q[1]);
 #pragma unroll
   for (int t = 0; t < 2; ++t) {
-    const int i = i0 + t;
+    const int i = w.a0 + t * w.W;
     if (i > M.n[0]) break;
-    const int64_t c = cidx(M, i, j, k), cw = cidx(W, i, j, k);
+    const int64_t c = cidx(M, i, w.j, w.k), cw = cidx(W, i, w.j, w.k);
     const double na = q0[c] + (double)e0[cw];
     const double nb = q1[c] + (double)e1[cw];
     q0[c] = na;
     q1[c] = nb;
-    if (M.wt && near_boundary(M, i, j, k, D)) write_through<double, D>(M, q0, q1, i, j, k, na, nb);
+    if (M.wt && near_boundary(M, i, w.j, w.k, D))
+      write_through<double, D>(M, q0, q1, i, w.j, w.k, na, nb);
   }
 }
 
