@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_relax(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
              const int* __restrict__ count, int color, TileRuns R) {
   const int n = *count;
+#pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) relax_item<T, D>(PT, items[b], color);
 }
 
@@ -93,6 +94,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_restrict(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                 const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+#pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];
     if (PT[it.patch].pprec == PREC_F32) restrict_item<TC, float, D>(PT, it);
@@ -106,6 +108,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, (sizeof(TC) == 4 ? 2 : 1) + (D 
     kb_coarse_load(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                    const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+#pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];
     if (PT[it.patch].pprec == PREC_F32) coarse_load_item<TC, float, D>(PT, it);
@@ -118,6 +121,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_correct(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+#pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];
     if (PT[it.patch].pprec == PREC_F32) correct_item<TC, float, D>(PT, it);
@@ -152,41 +156,45 @@ __global__ void __launch_bounds__(BLOCK_THREADS)
     kb_source(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
               const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+#pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) source_item<double, D>(PT, items[b], 1);
 }
 
 // FP64 form: residual partial of every master tile.
 template <int D>
-__global__ void __launch_bounds__(BLOCK_THREADS)
+__global__ void __launch_bounds__(BLOCK_THREADS, D == 2 ? 5 : 4)
     kb_resid(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
              const int* __restrict__ count, double* __restrict__ partials, TileRuns R) {
   const int n = *count;
-  for (int b = R.first(); b < n; b = R.next(b)) {
+  const WarpRuns w(R);
+#pragma unroll 1
+  for (int b = w.at; b < n; b = w.next(b)) {
     const Item it = items[b];
-    const DevPatch P = PT[it.patch];
-    if (!P.active) continue;  // uniform per CTA
-    const double s = block_sum(resid_item<double, D>(P, it));
-    if (threadIdx.x == 0 && threadIdx.y == 0) partials[b] = s;
+    const DevPatch& P = PT[it.patch];
+    if (!P.active) continue;
+    const double s = resid_rows<D>(P, it, [](int, int, int, bool, double2, double2, double2) {});
+    if (threadIdx.x == 0) partials[b] = s;
   }
 }
 
 // Mixed form: defect of every master tile (newstep_only = 0, with partials)
 // or of the masters starting a time step (newstep_only = 1: twin set-up only).
 template <int D>
-__global__ void __launch_bounds__(BLOCK_THREADS, BATCH_LATENCY_MIN_BLOCKS)
+__global__ void __launch_bounds__(BLOCK_THREADS, 4)
     kb_defect(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
               const int* __restrict__ count, double* __restrict__ partials, int newstep_only,
               TileRuns R) {
   const int n = *count;
-  for (int b = R.first(); b < n; b = R.next(b)) {
+  const WarpRuns w(R);
+#pragma unroll 1
+  for (int b = w.at; b < n; b = w.next(b)) {
     const Item it = items[b];
-    const DevPatch M = PT[it.patch];
-    if (!M.active || (newstep_only && !M.newstep)) continue;  // uniform per CTA
-    const bool w32 = PT[M.twin].prec == PREC_F32;
-    const double acc = w32 ? defect_item<float, D>(PT, it, newstep_only)
-                           : defect_item<double, D>(PT, it, newstep_only);
-    const double s = block_sum(acc);
-    if (!newstep_only && threadIdx.x == 0 && threadIdx.y == 0) partials[b] = s;
+    const DevPatch& M = PT[it.patch];
+    if (!M.active || (newstep_only && !M.newstep)) continue;
+    const DevPatch& W = PT[M.twin];
+    const double s = W.prec == PREC_F32 ? defect_rows<float, D>(M, W, it, !W.fused)
+                                        : defect_rows<double, D>(M, W, it, true);
+    if (!newstep_only && threadIdx.x == 0) partials[b] = s;
   }
 }
 
@@ -195,6 +203,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_update(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
               const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+#pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];
     if (PT[it.patch].prec == PREC_F32) update_item<float, D>(PT, it);
@@ -253,6 +262,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS)
     kb_filldown(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                 const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+#pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];
     if (!PT[it.patch].active) continue;

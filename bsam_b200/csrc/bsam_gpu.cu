@@ -506,19 +506,20 @@ void vcycle(bsam_gpu* h, int level) {
 void launch_resid(bsam_gpu* h) {
   const int nd = h->rp.ndims;
   const dim3 b = block_dim();
+  const unsigned g = (unsigned)(h->nmaster + TILE_Y - 1) / TILE_Y;
   if (!h->mixed) {
     if (nd == 2)
-      k_resid_norm<double, 2><<<h->nmaster, b, 0, h->stream>>>(
+      k_resid_norm<2><<<g, b, 0, h->stream>>>(
           h->d_patches, h->d_master, h->d_partials, h->d_status, h->nmaster, h->denom,
           h->rp.qerrortol);
     else
-      k_resid_norm<double, 3><<<h->nmaster, b, 0, h->stream>>>(
+      k_resid_norm<3><<<g, b, 0, h->stream>>>(
           h->d_patches, h->d_master, h->d_partials, h->d_status, h->nmaster, h->denom,
           h->rp.qerrortol);
   } else {
     const bool f32 = plan(h, h->finestlevel).prec == PREC_F32;
 #define DEFECT(TW, D)                                                                        \
-  k_defect<TW, D><<<h->nmaster, b, 0, h->stream>>>(h->d_patches, h->d_master, h->d_partials, \
+  k_defect<TW, D><<<g, b, 0, h->stream>>>(h->d_patches, h->d_master, h->d_partials, \
                                                    h->d_status, h->nmaster, h->denom,        \
                                                    h->rp.qerrortol)
     if (nd == 2) {

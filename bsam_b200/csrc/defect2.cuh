@@ -162,7 +162,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
             e0[cw] = 0.f;
             e1[cw] = 0.f;
             if (W.wt && near_boundary(W, i, j, 0, 2))
-              write_through<float, 2>(W, e0, e1, i, j, 0, 0.f, 0.f);
+              write_through_all<float, 2>(W, e0, e1, i, j, 0, 0.f, 0.f);
           }
         } else {
           double* e0 = fld<double>(W.q[0]);
@@ -173,7 +173,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
           e0[cw] = 0.0;
           e1[cw] = 0.0;
           if (W.wt && near_boundary(W, i, j, 0, 2))
-            write_through<double, 2>(W, e0, e1, i, j, 0, 0.0, 0.0);
+            write_through_all<double, 2>(W, e0, e1, i, j, 0, 0.0, 0.0);
         }
       }
     }

@@ -439,8 +439,8 @@ __device__ __forceinline__ void restrict_tile2(const DevPatch& C, const DevPatch
     ps0[pc] = v0;
     ps1[pc] = v1;
     if (R.wt && near_boundary(R, pi, pj, 0, 2)) {
-      write_through<TP, 2>(R, pq0, pq1, pi, pj, 0, v0, v1);
-      write_through<TP, 2>(R, ps0, ps1, pi, pj, 0, v0, v1);
+      write_through_all<TP, 2>(R, pq0, pq1, pi, pj, 0, v0, v1);
+      write_through_all<TP, 2>(R, ps0, ps1, pi, pj, 0, v0, v1);
     }
     if constexpr (DELTA)
       if (R.delta)
@@ -650,7 +650,7 @@ __global__ void __launch_bounds__(Fused2<T>::THREADS, MINB)
             m0[c] = na;
             m1[c] = nb;
             if (M.wt && near_boundary(M, i, j, 0, 2))
-              write_through<double, 2>(M, m0, m1, i, j, 0, na, nb);
+              write_through_all<double, 2>(M, m0, m1, i, j, 0, na, nb);
           }
         }
     } else {
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(Fused2<T>::THREADS, MINB)
             const T v0 = s0[srow + lx + d], v1 = s1[srow + lx + d];
             r0[i] = v0;
             r1[i] = v1;
-            if (P.wt && near_boundary(P, i, j, 0, 2)) write_through<T, 2>(P, o0, o1, i, j, 0, v0, v1);
+            if (P.wt && near_boundary(P, i, j, 0, 2)) write_through_all<T, 2>(P, o0, o1, i, j, 0, v0, v1);
           }
         }
     }

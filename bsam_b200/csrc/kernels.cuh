@@ -42,6 +42,22 @@ struct TileRuns {
   }
 };
 
+// The same for kernels whose warps take a tile each.
+struct WarpRuns {
+  int chunk, skip, at;
+  __device__ __forceinline__ WarpRuns(const TileRuns& R) {
+    const int w = (threadIdx.x + blockDim.x * threadIdx.y) / 32;
+    const int warps = blockDim.x * blockDim.y / 32;
+    chunk = R.chunk;
+    skip = ((int)gridDim.x * warps - 1) * chunk;
+    at = ((int)blockIdx.x * warps + w) * chunk;
+  }
+  __device__ __forceinline__ int next(int x) const {
+    ++x;
+    return (x % chunk) != 0 ? x : x + skip;
+  }
+};
+
 // The pre-smoothed state of a level: the second buffer when the level's
 // stages run the fused kernel (q -> qb -> q), else q itself.
 __device__ __forceinline__ void* const* mid_state(const DevPatch& P) {
@@ -122,11 +138,20 @@ __device__ __forceinline__ bool ghost_choice(int s, int co, int n, int lo_code, 
   return co == n && hi_code != BC_NONE;
 }
 
+// The one ghost of a dimension that coordinate co feeds, as its distance in that
+// dimension (0: none; 2 n + 1, which is none: two) and its face's code.
+__device__ __forceinline__ int ghost_step(int co, int n, int lo_code, int hi_code, int& code) {
+  const bool lo = lo_code == BC_PERIODIC ? co == n : co == 1 && lo_code != BC_NONE;
+  const bool hi = hi_code == BC_PERIODIC ? co == 1 : co == n && hi_code != BC_NONE;
+  code = lo ? lo_code : hi_code;
+  return lo && hi ? 2 * n + 1 : lo ? -co : hi ? n + 1 - co : 0;
+}
+
 // Ghost write-through for the cell (i,j,k) of patch P whose new values are
-// (v0, v1).
+// (v0, v1): every combination of the dimensions' choices.
 template <class T, int D>
-__device__ __forceinline__ void write_through(const DevPatch& P, T* q0, T* q1, int i, int j,
-                                              int k, T v0, T v1) {
+__device__ __forceinline__ void write_through_all(const DevPatch& P, T* q0, T* q1, int i, int j,
+                                                  int k, T v0, T v1) {
 #pragma unroll
   for (int sz = 0; sz < (D == 3 ? 3 : 1); ++sz) {
     int gz = k, cz = BC_NONE;
@@ -160,6 +185,31 @@ __device__ __forceinline__ void write_through(const DevPatch& P, T* q0, T* q1, i
       }
     }
   }
+}
+
+// The same, a cell that feeds one ghost through one face first: most of those that
+// feed any; cells at edges and corners go through all combinations.  (All through
+// the combinations: a colour pass of 128^3 23 us, now 20.9, of 48 x 32 x 40 FP32
+// 5.5, now 4.7.  As a loop over the ghosts a cell feeds, one by one: restriction of
+// 16^3 13.5 us against 9.7 and 8.2.  The 2D fused stages, which write few ghosts
+// and have no registers to spare, are 5 % slower this way: write_through_all.)
+template <class T, int D>
+__device__ __forceinline__ void write_through(const DevPatch& P, T* q0, T* q1, int i, int j,
+                                              int k, T v0, T v1) {
+  int cx, cy, cz = BC_NONE;
+  const int dx = ghost_step(i, P.n[0], P.bc[0], P.bc[1], cx);
+  const int dy = ghost_step(j, P.n[1], P.bc[2], P.bc[3], cy);
+  const int dz = D == 3 ? ghost_step(k, P.n[2], P.bc[4], P.bc[5], cz) : 0;
+  const int faces = (dx != 0) + (dy != 0) + (dz != 0);
+  if (faces == 0) return;
+  if (faces > 1 || dx > P.n[0] || dy > P.n[1] || (D == 3 && dz > P.n[2])) {
+    write_through_all<T, D>(P, q0, q1, i, j, k, v0, v1);
+    return;
+  }
+  const int code = dx ? cx : dy ? cy : cz;
+  const int64_t c = cidx(P, i + dx, j + dy, D == 3 ? k + dz : 0);
+  q0[c] = bc_map<T>(code, v0);
+  q1[c] = bc_map<T>(code, v1);
 }
 
 template <class T, int D>
@@ -516,26 +566,23 @@ __device__ __forceinline__ double block_sum(double v) {
   return s;  // valid in thread 0
 }
 
-// Second stage of a two-stage reduction: the last CTA to finish sums the
-// per-CTA partials in index order.  Returns true in thread 0 of that CTA
-// with the total in `total`.
-__device__ __forceinline__ bool last_block_total(double mine, double* partials,
-                                                 uint32_t* ticket, int nblocks,
-                                                 double& total) {
+// Second stage of a two-stage reduction over `count` partial sums that the CTAs
+// have stored (here: this CTA's by any of its threads): the last CTA to finish
+// sums them in index order.  Returns true in thread 0 of that CTA with the total
+// in `total`.
+__device__ __forceinline__ bool last_block_sum(const double* partials, uint32_t* ticket,
+                                               int nblocks, int count, double& total) {
   __shared__ bool is_last;
   const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
   const int nthreads = blockDim.x * blockDim.y * blockDim.z;
-  if (tid == 0) {
-    partials[blockIdx.x] = mine;
-    __threadfence();
-    const uint32_t t = atomicAdd(ticket, 1u);
-    is_last = (t == (uint32_t)nblocks - 1u);
-  }
+  __threadfence();
+  __syncthreads();
+  if (tid == 0) is_last = atomicAdd(ticket, 1u) == (uint32_t)nblocks - 1u;
   __syncthreads();
   if (!is_last) return false;
   __threadfence();
   double s = 0.0;
-  for (int b = tid; b < nblocks; b += nthreads) s += ((volatile double*)partials)[b];
+  for (int b = tid; b < count; b += nthreads) s += ((const volatile double*)partials)[b];
   const double tot = block_sum(s);
   if (tid == 0) {
     total = tot;
@@ -543,6 +590,14 @@ __device__ __forceinline__ bool last_block_total(double mine, double* partials,
     return true;
   }
   return false;
+}
+
+// The same with one partial sum per CTA, `mine` of thread 0.
+__device__ __forceinline__ bool last_block_total(double mine, double* partials,
+                                                 uint32_t* ticket, int nblocks,
+                                                 double& total) {
+  if (threadIdx.x + threadIdx.y + threadIdx.z == 0) partials[blockIdx.x] = mine;
+  return last_block_sum(partials, ticket, nblocks, nblocks, total);
 }
 
 // ---- tile bodies ---------------------------------------------------------------
@@ -567,29 +622,100 @@ __device__ __forceinline__ void relax_item(const DevPatch* __restrict__ PT, cons
   relax_cell<T, D>(P, i, w.j, w.k);
 }
 
-// Sum of rf^2 over this thread's cells of a tile (ErrorAFAS's SquareSum).
-template <class T, int D>
-__device__ __forceinline__ double resid_item(const DevPatch& P, const Item it) {
-  const int j = it.ty * TILE_Y + threadIdx.y + 1;
-  const int k = (D == 3) ? it.tz + 1 : 0;
-  const int i0 = (it.tx * 32 + threadIdx.x) * 2 + 1;
-  const T* q0 = fld<T>(P.q[0]);
-  const T* q1 = fld<T>(P.q[1]);
-  const T* f0 = fld<T>(P.f[0]);
-  const T* f1 = fld<T>(P.f[1]);
-  double acc = 0.0;
-  if (j <= P.n[1]) {
+// The residual of the FP64 cells of one TILE_X x TILE_Y tile by one warp, a pair
+// of cells a lane: out(i, j, k, two, r0, r1, q) for every pair inside (two: the
+// second cell is inside too; q: phi of both).  Returns the tile's sum of rf^2
+// (ErrorAFAS's SquareSum) in lane 0, in the order of block_sum with a thread per
+// pair: each row by the shuffle tree, then the rows in order.
+//
+// A row of q comes as aligned pairs, once for the three rows that read it; the
+// four rows' loads are independent of one another.  A CTA per tile, a thread per
+// pair and each operand loaded where it is used, kept L1 at 76 % and memory at 28 %
+// of their rates: the norm of 128^3 45 us, now 30.5; the defect (mixed.cuh) of
+// 96 x 64 x 80 24 us, now 17, and of 24 masters of 32^3 and 64^3 154 us, now 110.
+// (In 2D the norm of 96 masters takes 38 us either way.)
+template <int D, class Out>
+__device__ __forceinline__ double resid_rows(const DevPatch& P, const Item it, Out&& out) {
+  const int lane = threadIdx.x & 31;
+  const int i0 = it.tx * TILE_X + 2 * lane + 1, j0 = it.ty * TILE_Y + 1;
+  const int k = D == 3 ? it.tz + 1 : 0;
+  const bool on = i0 <= P.n[0], two = i0 < P.n[0];
+  const int rows = min(TILE_Y, P.n[1] - j0 + 1);
+  double acc[TILE_Y];
 #pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      const int i = i0 + t;
-      if (i <= P.n[0]) {
-        T r0, r1;
-        residual_cell<T, D>(P, q0, q1, f0, f1, cidx(P, i, j, k), r0, r1);
-        acc += (double)r0 * (double)r0 + (double)r1 * (double)r1;
+  for (int r = 0; r < TILE_Y; ++r) acc[r] = 0.0;
+  if (on) {
+    const int64_t c0 = cidx(P, i0, j0, k);
+    const double* q0 = fld<double>(P.q[0]) + c0;
+    const double* q1 = fld<double>(P.q[1]) + c0;
+    const double* f0 = fld<double>(P.f[0]) + c0;
+    const double* f1 = fld<double>(P.f[1]) + c0;
+    double2 a[2][TILE_Y + 2];  // rows j0 - 1 ... j0 + TILE_Y of the pair
+#pragma unroll
+    for (int r = 0; r < TILE_Y + 2; ++r)
+      if (r <= rows + 1) {
+        a[0][r] = load_pair<double>(q0 + (r - 1) * P.sy);
+        a[1][r] = load_pair<double>(q1 + (r - 1) * P.sy);
       }
+#pragma unroll
+    for (int r = 0; r < TILE_Y; ++r) {
+      if (r >= rows) break;
+      const int64_t o = r * P.sy;
+      const double2 g0 = load_pair<double>(f0 + o), g1 = load_pair<double>(f1 + o);
+      Problem::Stencil<double, D> lo, hi;
+      lo.pc = a[0][r + 1].x;
+      lo.mc = a[1][r + 1].x;
+      hi.pc = a[0][r + 1].y;
+      hi.mc = a[1][r + 1].y;
+      lo.pm[0] = q0[o - 1];
+      lo.mm[0] = q1[o - 1];
+      lo.pp[0] = hi.pc;
+      lo.mp[0] = hi.mc;
+      hi.pm[0] = lo.pc;
+      hi.mm[0] = lo.mc;
+      hi.pp[0] = two ? q0[o + 2] : 0.0;
+      hi.mp[0] = two ? q1[o + 2] : 0.0;
+      lo.pm[1] = a[0][r].x;
+      lo.mm[1] = a[1][r].x;
+      lo.pp[1] = a[0][r + 2].x;
+      lo.mp[1] = a[1][r + 2].x;
+      hi.pm[1] = a[0][r].y;
+      hi.mm[1] = a[1][r].y;
+      hi.pp[1] = a[0][r + 2].y;
+      hi.mp[1] = a[1][r + 2].y;
+      if (D == 3) {
+        const double2 zm0 = load_pair<double>(q0 + o - P.sz), zp0 = load_pair<double>(q0 + o + P.sz);
+        const double2 zm1 = load_pair<double>(q1 + o - P.sz), zp1 = load_pair<double>(q1 + o + P.sz);
+        lo.pm[D - 1] = zm0.x;
+        lo.pp[D - 1] = zp0.x;
+        lo.mm[D - 1] = zm1.x;
+        lo.mp[D - 1] = zp1.x;
+        hi.pm[D - 1] = zm0.y;
+        hi.pp[D - 1] = zp0.y;
+        hi.mm[D - 1] = zm1.y;
+        hi.mp[D - 1] = zp1.y;
+      }
+      double o0, o1;
+      double2 r0, r1;
+      Problem::OperatorCell<double, D>(lo, P.tmp1, P.tmp2, P.alpha, o0, o1);
+      r0.x = g0.x - o0;
+      r1.x = g1.x - o1;
+      Problem::OperatorCell<double, D>(hi, P.tmp1, P.tmp2, P.alpha, o0, o1);
+      r0.y = g0.y - o0;
+      r1.y = g1.y - o1;
+      acc[r] = r0.x * r0.x + r1.x * r1.x;
+      if (two) acc[r] += r0.y * r0.y + r1.y * r1.y;
+      out(i0, j0 + r, k, two, r0, r1, a[0][r + 1]);
     }
   }
-  return acc;
+  double s = 0.0;
+#pragma unroll
+  for (int r = 0; r < TILE_Y; ++r) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[r] += __shfl_down_sync(0xffffffffu, acc[r], o);
+    s += acc[r];
+  }
+  return s;
 }
 
 template <class TC, class TP, int D>
@@ -673,15 +799,20 @@ __global__ void __launch_bounds__(BLOCK_THREADS)
 
 // ErrorAFAS / L2Error / SquareSum (afas:108-221), errortype 1:
 // residual = sqrt(sum rf^2 / (nrvars * ncells)) over the finest level.
-template <class T, int D>
-__global__ void __launch_bounds__(BLOCK_THREADS)
+template <int D>
+__global__ void __launch_bounds__(BLOCK_THREADS, D == 2 ? 5 : 4)
     k_resid_norm(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                  double* __restrict__ partials, DevStatus* __restrict__ st, int nitems,
                  double denom, double tol) {
-  const Item it = items[blockIdx.x];
-  const double bs = block_sum(resid_item<T, D>(PT[it.patch], it));
+  const int b = blockIdx.x * TILE_Y + threadIdx.y;  // a tile per warp
+  if (b < nitems) {
+    const Item it = items[b];
+    const double s = resid_rows<D>(PT[it.patch], it,
+                                   [](int, int, int, bool, double2, double2, double2) {});
+    if (threadIdx.x == 0) partials[b] = s;
+  }
   double total;
-  if (last_block_total(bs, partials, &st->ticket, nitems, total)) {
+  if (last_block_sum(partials, &st->ticket, gridDim.x, nitems, total)) {
     const double r = sqrt(total / denom);
     st->sumsq = total;
     st->residual = r;

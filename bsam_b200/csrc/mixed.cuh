@@ -22,46 +22,54 @@
 
 namespace bsam {
 
-// Defect of one master tile: ErrorAFAS of q64 (the same norm as
+// Defect of one master tile by one warp: ErrorAFAS of q64 (the same norm as
 // k_resid_norm) plus the twin's start (e = 0), base and right-hand side.
-// Returns this thread's sum of squares.  newstep_only (batches): only masters
-// whose time step starts in this iteration.
+// Returns the tile's sum of squares in lane 0.  zero: e = 0 is stored (a batch's
+// fused stage starts from it without reading it).
 template <class TW, int D>
-__device__ __forceinline__ double defect_item(const DevPatch* __restrict__ PT, const Item it,
-                                              int newstep_only) {
-  const DevPatch M = PT[it.patch];
-  if (!M.active || (newstep_only && !M.newstep)) return 0.0;
-  const DevPatch W = PT[M.twin];
-  const int j = it.ty * TILE_Y + threadIdx.y + 1;
-  const int k = (D == 3) ? it.tz + 1 : 0;
-  const int i0 = (it.tx * 32 + threadIdx.x) * 2 + 1;
-  const double* q0 = fld<double>(M.q[0]);
-  const double* q1 = fld<double>(M.q[1]);
-  const double* f0 = fld<double>(M.f[0]);
-  const double* f1 = fld<double>(M.f[1]);
+__device__ __forceinline__ double defect_rows(const DevPatch& M, const DevPatch& W, const Item it,
+                                              bool zero) {
+  using V = typename PairOf<TW>::V;
   TW* e0 = fld<TW>(W.q[0]);
   TW* e1 = fld<TW>(W.q[1]);
-  double acc = 0.0;
-  if (j <= M.n[1]) {
-#pragma unroll
-    for (int t = 0; t < 2; ++t) {
-      const int i = i0 + t;
-      if (i > M.n[0]) break;
-      const int64_t c = cidx(M, i, j, k);
-      double r0, r1;
-      residual_cell<double, D>(M, q0, q1, f0, f1, c, r0, r1);
-      acc += r0 * r0 + r1 * r1;
-      const int64_t cw = cidx(W, i, j, k);
-      fld<TW>(W.f[0])[cw] = TW(r0);
-      fld<TW>(W.f[1])[cw] = TW(r1);
-      fld<TW>(W.bs)[cw] = TW(q0[c]);
-      e0[cw] = TW(0);
-      e1[cw] = TW(0);
-      if (W.wt && near_boundary(W, i, j, k, D))
-        write_through<TW, D>(W, e0, e1, i, j, k, TW(0), TW(0));
-    }
-  }
-  return acc;
+  TW* f0 = fld<TW>(W.f[0]);
+  TW* f1 = fld<TW>(W.f[1]);
+  TW* bs = fld<TW>(W.bs);
+  return resid_rows<D>(
+      M, it, [&](int i, int j, int k, bool two, double2 r0, double2 r1, double2 q) {
+        const int64_t c = cidx(W, i, j, k);
+        if (two) {
+          auto put = [&](TW* p, TW x, TW y) { *reinterpret_cast<V*>(p + c) = V{x, y}; };
+          put(f0, TW(r0.x), TW(r0.y));
+          put(f1, TW(r1.x), TW(r1.y));
+          put(bs, TW(q.x), TW(q.y));
+          if (zero) {
+            put(e0, TW(0), TW(0));
+            put(e1, TW(0), TW(0));
+          }
+        } else {
+          f0[c] = TW(r0.x);
+          f1[c] = TW(r1.x);
+          bs[c] = TW(q.x);
+          if (zero) e0[c] = e1[c] = TW(0);
+        }
+        if (!zero || !W.wt) return;
+        // Ghosts across the faces; those across two or three are not read here (no
+        // patch has its parent on the finest level).
+        auto ghost = [&](int64_t g, int code, bool pair) {
+          const TW z = bc_map<TW>(code, TW(0));
+          e0[g] = e1[g] = z;
+          if (pair) e0[g + 1] = e1[g + 1] = z;
+        };
+        if (i == 1) ghost(c - 1, W.bc[0], false);
+        if (i + (int)two == W.n[0]) ghost(c + 1 + (int)two, W.bc[1], false);
+        if (j == 1) ghost(c - W.sy, W.bc[2], two);
+        if (j == W.n[1]) ghost(c + W.sy, W.bc[3], two);
+        if (D == 3) {
+          if (k == 1) ghost(c - W.sz, W.bc[4], two);
+          if (k == W.n[2]) ghost(c + W.sz, W.bc[5], two);
+        }
+      });
 }
 
 // q64 += e on one work tile of a twin; ghosts by write-through.
@@ -92,13 +100,19 @@ __device__ __forceinline__ void update_item(const DevPatch* __restrict__ PT, con
 
 // Defect kernel over the masters' tiles, with the FP64 norm in d_status.
 template <class TW, int D>
-__global__ void __launch_bounds__(BLOCK_THREADS)
+__global__ void __launch_bounds__(BLOCK_THREADS, 4)
     k_defect(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
              double* __restrict__ partials, DevStatus* __restrict__ st, int nitems,
              double denom, double tol) {
-  const double bs = block_sum(defect_item<TW, D>(PT, items[blockIdx.x], 0));
+  const int b = blockIdx.x * TILE_Y + threadIdx.y;  // a tile per warp
+  if (b < nitems) {
+    const Item it = items[b];
+    const DevPatch& M = PT[it.patch];
+    const double s = defect_rows<TW, D>(M, PT[M.twin], it, true);
+    if (threadIdx.x == 0) partials[b] = s;
+  }
   double total;
-  if (last_block_total(bs, partials, &st->ticket, nitems, total)) {
+  if (last_block_sum(partials, &st->ticket, gridDim.x, nitems, total)) {
     const double r = sqrt(total / denom);
     st->sumsq = total;
     st->residual = r;
