@@ -38,6 +38,7 @@
 
 #include "../../include/bsam_batch.h"
 #include "batch.cuh"
+#include "chain.cuh"
 #include "bsam_types.h"
 #include "defect2.cuh"
 #include "engine_view.h"
@@ -77,7 +78,8 @@ enum {
   L_CORR = 2 + 3 * MAXD,
   L_RESTR = 2 + 4 * MAXD,
   L_UPD = 2 + 5 * MAXD,
-  NLIST = 3 + 5 * MAXD
+  L_CHAIN = 3 + 5 * MAXD,  // tops of the bottom chains that fit in shared memory
+  NLIST = 4 + 5 * MAXD
 };
 
 // Lists of the refined hierarchies (SLOT_AMR), over the records of their own
@@ -95,7 +97,8 @@ enum {
   A_GHOST = 2 + 3 * (MAXD + 1),
   A_SNAP = 2 + 4 * (MAXD + 1),
   A_CORR = 2 + 5 * (MAXD + 1),
-  ANLIST = 2 + 6 * (MAXD + 1)
+  A_CHAIN = 2 + 6 * (MAXD + 1),
+  ANLIST = 3 + 6 * (MAXD + 1)
 };
 
 struct List {
@@ -195,6 +198,7 @@ struct bsam_batch {
   // graph
   cudaGraphExec_t exec = nullptr;
   int cap_depth = 0;
+  size_t chain_smem = 0;  // shared memory of the largest bottom chain so far
   bool need_capture = true;
   int64_t kernels_per_tick = 0;
   bsam_batch_stats st{};
@@ -573,6 +577,20 @@ int plan_slot(bsam_batch* b, const bsam_batch_problem* pr, int rec0, char* base,
 }
 
 // Appends a slot's tiles to the lists and records its master range.
+// Does a bottom chain of these extents, top first, fit in a CTA's shared memory
+// (chain.cuh)?  Keeps the largest size so far.
+bool chain_fits(bsam_batch* b, const std::vector<std::array<int, 3>>& n, bool delta) {
+  ChainPlan C;
+  if (!chain_layout(b->bp.ndims, n, std::vector<int>(n.size(), PREC_F64), delta,
+                    b->bp.nsmoothingpasses, 1, false, C))
+    return false;
+  if (C.smem > b->chain_smem) {
+    b->chain_smem = C.smem;
+    b->need_capture = true;
+  }
+  return true;
+}
+
 void append_items(bsam_batch* b, int s) {
   SlotPlan& S = b->slots[s];
   const int nd = b->bp.ndims;
@@ -583,7 +601,13 @@ void append_items(bsam_batch* b, int s) {
   C.ie = (int)b->lists[L_MASTER].h.size();
   if (b->mixed && !S.recs[1].fused)
     work_tiles(rec0 + 1, S.recs[1].n, nd, b->lists[L_UPD].h);
-  b->lists[L_TOPS].h.push_back(Item{S.top, 0, 0, 0});
+  {
+    std::vector<std::array<int, 3>> n;
+    for (int r = S.top - rec0; r < S.nrec; ++r)
+      n.push_back({S.recs[r].n[0], S.recs[r].n[1], S.recs[r].n[2]});
+    const bool fits = chain_fits(b, n, b->mixed);
+    b->lists[fits ? L_CHAIN : L_TOPS].h.push_back(Item{S.top, 0, 0, 0});
+  }
   const int first = b->mixed ? 1 : 0;  // record of depth 0
   for (int d = 0; d < S.ntop; ++d) {
     const int r = first + d;
@@ -687,7 +711,14 @@ void amr_append(bsam_batch* b, int s, bool active) {
   C.ib = (int)LA[A_MASTER].h.size();
   for (int p : V.masters) tiles_for(r0 + p, V.recs[p].n, nd, LA[A_MASTER].h);
   C.ie = (int)LA[A_MASTER].h.size();
-  LA[A_TOPS].h.push_back(Item{r0 + V.levels[S.chain - V.minlevel].patches[0], 0, 0, 0});
+  {
+    const int top = V.levels[S.chain - V.minlevel].patches[0];
+    std::vector<std::array<int, 3>> n;
+    for (int r = top; r >= 0; r = V.recs[r].parent)
+      n.push_back({V.recs[r].n[0], V.recs[r].n[1], V.recs[r].n[2]});
+    const bool fits = chain_fits(b, n, false);
+    LA[fits ? A_CHAIN : A_TOPS].h.push_back(Item{r0 + top, 0, 0, 0});
+  }
   for (int l = V.finestlevel; l >= S.chain; --l) {
     const EngineLevelView& E = V.levels[l - V.minlevel];
     const int d = V.finestlevel - l;
@@ -1015,12 +1046,33 @@ void tick_t(bsam_batch* b, cudaGraphConditionalHandle handle, int in_graph) {
     ++n;
   }
   {
-    const int cap = std::max(1, L[L_TOPS].cap);
-    const int gb = std::max(1, std::min(cap, 4 * b->nsm));
-    kb_bottom<D><<<gb, BATCH_BOTTOM_THREADS, 0, s>>>(pt, L[L_TOPS].d, cnt + L_TOPS, nu);
-    ++n;
+    // Bottom chains: in shared memory (two CTAs per SM by their registers), the
+    // others in global memory.
+    auto chains = [&](auto k, const DevPatch* table, const List& T, const int* count, int all) {
+      if (T.cap == 0) return;
+      cudaLaunchConfig_t cfg{};
+      cfg.gridDim = dim3((unsigned)std::min(T.cap, 2 * b->nsm));
+      cfg.blockDim = dim3(BATCH_CHAIN_THREADS);
+      cfg.dynamicSmemBytes = b->chain_smem;
+      cfg.stream = s;
+      cudaLaunchAttribute at{};
+      at.id = cudaLaunchAttributeClusterDimension;
+      at.val.clusterDim.x = at.val.clusterDim.y = at.val.clusterDim.z = 1;
+      cfg.attrs = &at;
+      cfg.numAttrs = 1;
+      (void)cudaLaunchKernelEx(&cfg, k, table, (const Item*)T.d, count, nu, all);
+      ++n;
+    };
+    if (b->mixed) chains(kb_chain<D, true>, pt, L[L_CHAIN], cnt + L_CHAIN, 0);
+    else chains(kb_chain<D, false>, pt, L[L_CHAIN], cnt + L_CHAIN, 0);
+    chains(kb_chain<D, false>, apt, LA[A_CHAIN], acnt + A_CHAIN, 1);
+    if (L[L_TOPS].cap > 0) {
+      const int gb = std::min(L[L_TOPS].cap, 4 * b->nsm);
+      kb_bottom<D><<<gb, BATCH_BOTTOM_THREADS, 0, s>>>(pt, L[L_TOPS].d, cnt + L_TOPS, nu);
+      ++n;
+    }
     if (LA[A_TOPS].cap > 0) {
-      const int ga = std::max(1, std::min(LA[A_TOPS].cap, 4 * b->nsm));
+      const int ga = std::min(LA[A_TOPS].cap, 4 * b->nsm);
       kb_bottom<D><<<ga, BATCH_BOTTOM_THREADS, 0, s>>>(apt, LA[A_TOPS].d, acnt + A_TOPS, nu);
       ++n;
     }
@@ -1349,6 +1401,13 @@ int bsam_batch_create(bsam_batch** out, int device, const bsam_batch_params* p) 
          cudaFuncSetAttribute(kb_smooth2<double, false, 2, 2>,
                               cudaFuncAttributeMaxDynamicSharedMemorySize,
                               (int)(2 * Fused2<double>::smem(false))) == cudaSuccess;
+  auto chain_attr = [](auto k) {
+    return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)CHAIN_SMEM_MAX) == cudaSuccess;
+  };
+  if (ok)
+    ok = chain_attr(kb_chain<2, true>) && chain_attr(kb_chain<2, false>) &&
+         chain_attr(kb_chain<3, true>) && chain_attr(kb_chain<3, false>);
   if (!ok) {
     cudaGetLastError();
     bsam_batch_destroy(b);

@@ -631,7 +631,7 @@ template <class T, class TP, int D, bool DELTA, bool SLAB, bool SINGLE>
 __device__ __forceinline__ void chain_visit_pairs(const ChainCtx& X, int l, bool up, bool raw,
                                                   const ChainLevel& L, const ChainSlab& S,
                                                   const ChainLevel& P, ChainSync<SLAB> sync) {
-  const int nt = SLAB ? CHAIN_THREADS : 32 * sync.warps;
+  const int nt = SLAB ? (int)blockDim.x : 32 * sync.warps;
   ChainPair<T, D> R;
   R.on = false;
   auto load = [&](int idx) {
@@ -694,7 +694,7 @@ template <class T, int D, bool DELTA, bool SLAB>
 __device__ __forceinline__ void chain_visit_cells(const ChainCtx& X, int l, bool raw,
                                                   const ChainLevel& L, const ChainSlab& S,
                                                   ChainSync<SLAB> sync) {
-  const int nt = SLAB ? CHAIN_THREADS : 32 * sync.warps;
+  const int nt = SLAB ? (int)blockDim.x : 32 * sync.warps;
   const int w = L.n[0], h = D == 3 ? L.n[1] : 1, total = w * h * S.nr;
   const bool single = total <= nt;
   ChainCell<T, D> C;
@@ -743,7 +743,7 @@ __device__ __noinline__ void chain_visit_t(const ChainCtx& X, int l, bool up, bo
   const ChainSlab S = X.S[l];
   const bool last = l + 1 == X.PL->nlev;
   const int cells = L.n[0] * (D == 3 ? L.n[1] : 1) * S.nr, work = last ? cells : cells >> 1;
-  const ChainSync<SLAB> sync{min(max((work + 31) / 32, 1), CHAIN_THREADS / 32)};
+  const ChainSync<SLAB> sync{min(max((work + 31) / 32, 1), (int)blockDim.x / 32)};
   if (!SLAB && (int)threadIdx.x >= 32 * sync.warps) {
     __syncthreads();
     return;
@@ -752,7 +752,7 @@ __device__ __noinline__ void chain_visit_t(const ChainCtx& X, int l, bool up, bo
     chain_visit_cells<T, D, DELTA, SLAB>(X, l, raw, L, S, sync);
   } else {
     const ChainLevel& P = X.PL->L[l + 1];
-    if (work <= CHAIN_THREADS)
+    if (work <= (int)blockDim.x)
       chain_visit_pairs<T, TP, D, DELTA, SLAB, true>(X, l, up, raw, L, S, P, sync);
     else
       chain_visit_pairs<T, TP, D, DELTA, SLAB, false>(X, l, up, raw, L, S, P, sync);
@@ -872,7 +872,7 @@ __device__ __forceinline__ void chain_load_top(const DevPatch& G, const ChainLev
   const int ex = L.n[0] + 2, ey = D == 3 ? L.n[1] + 2 : 1;
   auto copy = [&](uint32_t dst, const T* s0, const T* s1, int rows, int first) {
     const int total = ex * ey * rows;
-    for (int e = threadIdx.x; e < total; e += CHAIN_THREADS) {
+    for (int e = threadIdx.x; e < total; e += blockDim.x) {
       const int r = e / ex, i = e - r * ex;
       const int t = D == 3 ? r / ey : r, j = D == 3 ? r - t * ey : 0;
       const int64_t g = i + (D == 3 ? j * G.sy : 0) + (first + t) * gs;
@@ -908,7 +908,7 @@ __device__ __forceinline__ void chain_store(const DevPatch& G, const ChainLevel&
     if (x >= 1 && x <= n) return x;
     return (x == 0) == (code == BC_PERIODIC) ? n : 1;
   };
-  for (int e = threadIdx.x; e < ex * ey * (t1 - t0 + 1); e += CHAIN_THREADS) {
+  for (int e = threadIdx.x; e < ex * ey * (t1 - t0 + 1); e += blockDim.x) {
     const int i = e % ex, r = e / ex;
     const int j = D == 3 ? r % ey : 0, t = t0 + (D == 3 ? r / ey : r);
     int cx, cy = BC_COPY, ct = BC_COPY;
@@ -1016,6 +1016,112 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
     else chain_store<double, D>(W, PL.L[l], slabs[l], l > 0);
   }
   chain_cluster_sync();  // no CTA leaves while another may still read its memory
+}
+
+// ---- chains of a batch, a CTA each ---------------------------------------------------
+
+// Lays out the FP64 chain from record `top` down its parent links in this CTA's
+// shared memory, as chain_layout does for one CTA, and fills in the records'
+// faces and constants; a level per lane of the first warp.  (From the host it
+// would be 2 KB for every problem admitted.)
+template <int D, bool DELTA>
+__device__ __forceinline__ void chain_plan(const DevPatch* __restrict__ PT, int top, int nu,
+                                           ChainPlan& PL, ChainSlab* slabs) {
+  if (threadIdx.x >= 32) return;
+  const int l = threadIdx.x;
+  int p = l < CHAIN_MAX_LEVELS ? top : -1;
+  for (int s = 0; s < l && p >= 0; ++s) p = PT[p].parent;
+  const unsigned levels = __ballot_sync(0xffffffffu, p >= 0);
+  const DevPatch& P = PT[max(p, 0)];
+  const int n0 = P.n[0], n1 = P.n[1], ns = P.n[D - 1];
+  const int pitch = n0 + 2, sstr = D == 3 ? pitch * (n1 + 2) : pitch;
+  const uint32_t q = 16u * (uint32_t)((ns + 2) * sstr), f = 16u * (uint32_t)(ns * sstr);
+  const uint32_t b = DELTA ? (8u * (uint32_t)(ns * sstr) + 15u) / 16u * 16u : 0u;
+  const uint32_t mine = p >= 0 ? q + f + (l > 0 ? q : 0u) + b : 0u;
+  uint32_t end = mine;
+#pragma unroll
+  for (int o = 1; o < 32; o *= 2) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, end, o);
+    if (l >= o) end += x;
+  }
+  if (l == 0) {
+    PL.nlev = __popc(levels);
+    PL.nslab = 0;
+    PL.nu = nu;
+    PL.ctas = 1;
+  }
+  if (p < 0) return;
+  ChainLevel& L = PL.L[l];
+  L.patch = p;
+  L.n[0] = n0;
+  L.n[1] = n1;
+  L.n[2] = P.n[2];
+  L.ns = ns;
+  L.pitch = pitch;
+  L.sstr = sstr;
+  L.prec = PREC_F64;
+  L.delta = DELTA ? 1 : 0;
+  int maps = 0;
+#pragma unroll
+  for (int face = 0; face < 6; ++face) {
+    const int code = P.bc[face];
+    L.bc[face] = code;
+    if (face < 2 * D && (code == BC_REFLECT || code == BC_NEGATE)) maps = 1;
+  }
+  L.maps = maps;
+  auto magic = [](uint32_t d) { return d == 1u ? 0u : 0xffffffffu / d + 1u; };
+  L.w = (uint32_t)max(1, n0 / 2);
+  L.h = (uint32_t)(D == 3 ? max(1, n1 / 2) : 1);
+  L.mw = magic(L.w);
+  L.mh = magic(L.h);
+  L.active = 1;
+  L.units = ns % 2 ? ns : ns / 2;
+  L.q = chain_base() + end - mine;
+  L.f = L.q + q;
+  L.qs = l > 0 ? L.f + f : 0u;
+  L.bs = L.f + f + (l > 0 ? q : 0u);
+  L.tmp1 = P.tmp1;
+  L.tmp2 = P.tmp2;
+  L.tmp3 = P.tmp3;
+  L.alpha = P.alpha;
+  ChainSlab S{};
+  S.lo = 1;
+  S.nr = ns;
+  S.lo_r = S.hi_r = -1;
+  slabs[l] = S;
+}
+
+// AFASVcycle of bottom chains that fit in a CTA's shared memory, a CTA per chain
+// at a time.  DELTA: correction-form levels.  all: every level's fields go back
+// to global memory, not only the top's state.
+// In global memory (bottom.cuh) a chain is some 60 phases of about 1.4 us each
+// whose loads wait on L2: 96 chains of 32^2 and below took 85 us, now 41; 24 of
+// 8^3 and below 128, now 41; 512 of 32^2 in correction form, two CTAs of 256
+// threads per SM in two waves, 127, now 96.
+constexpr int BATCH_CHAIN_THREADS = 256;
+template <int D, bool DELTA>
+__global__ void __launch_bounds__(BATCH_CHAIN_THREADS, 2)
+    kb_chain(const DevPatch* __restrict__ PT, const Item* __restrict__ tops,
+             const int* __restrict__ count, int nu, int all) {
+  __shared__ ChainPlan PL;
+  __shared__ ChainSlab slabs[CHAIN_MAX_LEVELS];
+  const int n = *count;
+  for (int b = blockIdx.x; b < n; b += gridDim.x) {
+    const int top = tops[b].patch;
+    if (!PT[top].active) continue;  // uniform per CTA
+    __syncthreads();  // the previous chain's memory is no longer read
+    chain_plan<D, DELTA>(PT, top, nu, PL, slabs);
+    __syncthreads();
+    chain_load_top<double, D>(PT[top], PL.L[0], slabs[0]);
+    __syncthreads();
+    const ChainCtx X{&PL, slabs, 0};
+    for (int l = 0; l < PL.nlev; ++l)
+      chain_visit_t<double, double, D, DELTA, false>(X, l, false, l == 0);
+    for (int l = PL.nlev - 2; l >= 0; --l)
+      chain_visit_t<double, double, D, DELTA, false>(X, l, true, false);
+    for (int l = 0; l < (all ? PL.nlev : 1); ++l)
+      chain_store<double, D>(PT[PL.L[l].patch], PL.L[l], slabs[l], l > 0);
+  }
 }
 
 // ---- host side -------------------------------------------------------------------
