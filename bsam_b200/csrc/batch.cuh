@@ -79,10 +79,11 @@ struct BatchCtl {
 };
 
 template <class T, int D>
-__global__ void __launch_bounds__(BLOCK_THREADS, 8)
+__global__ void __launch_bounds__(BLOCK_THREADS)
     kb_relax(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
              const int* __restrict__ count, int color, TileRuns R) {
   const int n = *count;
+  R = R.fit(n);
 #pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) relax_item<T, D>(PT, items[b], color);
 }
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_restrict(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                 const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+  R = R.fit(n);
 #pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];
@@ -108,6 +110,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, (sizeof(TC) == 4 ? 2 : 1) + (D 
     kb_coarse_load(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                    const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+  R = R.fit(n);
 #pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];
@@ -121,6 +124,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_correct(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+  R = R.fit(n);
 #pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];
@@ -156,6 +160,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS)
     kb_source(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
               const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+  R = R.fit(n);
 #pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) source_item<double, D>(PT, items[b], 1);
 }
@@ -166,7 +171,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, D == 2 ? 5 : 4)
     kb_resid(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
              const int* __restrict__ count, double* __restrict__ partials, TileRuns R) {
   const int n = *count;
-  const WarpRuns w(R);
+  const WarpRuns w(R, n);
 #pragma unroll 1
   for (int b = w.at; b < n; b = w.next(b)) {
     const Item it = items[b];
@@ -185,7 +190,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4)
               const int* __restrict__ count, double* __restrict__ partials, int newstep_only,
               TileRuns R) {
   const int n = *count;
-  const WarpRuns w(R);
+  const WarpRuns w(R, n);
 #pragma unroll 1
   for (int b = w.at; b < n; b = w.next(b)) {
     const Item it = items[b];
@@ -203,6 +208,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
     kb_update(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
               const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+  R = R.fit(n);
 #pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];
@@ -262,6 +268,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS)
     kb_filldown(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                 const int* __restrict__ count, TileRuns R) {
   const int n = *count;
+  R = R.fit(n);
 #pragma unroll 1
   for (int b = R.first(); b < n; b = R.next(b)) {
     const Item it = items[b];

@@ -57,13 +57,10 @@ constexpr int DEFAULT_BOTTOM_CELLS = 1024;
 // Default runs of consecutive list entries per CTA visit (TileRuns) for the
 // small-tile list kernels and for the fused stages (tuning.tile_chunk and
 // tuning.fused_chunk; 1 = grid-stride order).
-// One tile a visit: with runs of two the short lists of the coarse levels kept
-// half as many CTAs busy (24 problems of 32^3 and 64^3 20.8 -> 19.4 ms, 96 of
-// 64^2 to 256^2 22.2 -> 21.8, 512 of them the same).
-constexpr int kDefaultTileChunk = 1;
+constexpr int kDefaultTileChunk = 2;
 constexpr int kDefaultFusedChunk = 1;
 // Runs of the staged defect, in units of tile_chunk.
-constexpr int kDefectRunFactor = 8;
+constexpr int kDefectRunFactor = 4;
 // Lists: master tiles (sums); bottom-chain tops; per top depth d: footprint
 // tiles (coarse load), tiles of records smoothed per colour pass, fused-stage
 // tiles, blocks of records corrected and footprint tiles of records restricted

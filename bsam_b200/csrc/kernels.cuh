@@ -32,9 +32,16 @@ template <class T> __device__ __forceinline__ T* fld(void* p) { return static_ca
 // plain grid-stride order).  A list holds each problem's tiles in a row, so
 // the tiles of a run mostly share their patch records, which after the
 // run's first tile come from L1 instead of a chain of L2 round trips; the
-// order in which a CTA visits tiles changes no result.
+// order in which a CTA visits tiles changes no result.  A list too short to
+// give every CTA a run is taken tile by tile (fit): in runs of two the coarse
+// levels' lists kept half as many CTAs busy (24 problems of 32^3 and 64^3 20.8
+// ms, tile by tile 19.4; but colour passes of the finest level 37 and 43 us).
 struct TileRuns {
   int chunk;
+  __device__ __forceinline__ TileRuns fit(int n, int takers) const {
+    return TileRuns{n >= takers * chunk ? chunk : 1};
+  }
+  __device__ __forceinline__ TileRuns fit(int n) const { return fit(n, (int)gridDim.x); }
   __device__ __forceinline__ int first() const { return (int)blockIdx.x * chunk; }
   __device__ __forceinline__ int next(int x) const {
     ++x;
@@ -45,10 +52,10 @@ struct TileRuns {
 // The same for kernels whose warps take a tile each.
 struct WarpRuns {
   int chunk, skip, at;
-  __device__ __forceinline__ WarpRuns(const TileRuns& R) {
+  __device__ __forceinline__ WarpRuns(const TileRuns& R, int n) {
     const int w = (threadIdx.x + blockDim.x * threadIdx.y) / 32;
     const int warps = blockDim.x * blockDim.y / 32;
-    chunk = R.chunk;
+    chunk = R.fit(n, (int)gridDim.x * warps).chunk;
     skip = ((int)gridDim.x * warps - 1) * chunk;
     at = ((int)blockIdx.x * warps + w) * chunk;
   }
