@@ -368,6 +368,7 @@ __device__ __forceinline__ void ghost2_patch(const DevPatch* __restrict__ PT, in
 static __global__ void k_ghost2(const DevPatch* __restrict__ PT, const int* __restrict__ patches,
                          const OverlapCopy* __restrict__ cps, const int2* __restrict__ ranges,
                          int ipass) {
+  after_previous();
   ghost2_patch(PT, patches[blockIdx.x], cps, ranges[blockIdx.x], ipass);
 }
 
@@ -411,6 +412,7 @@ __device__ __forceinline__ void ghost3_patch(const DevPatch* __restrict__ PT, in
 static __global__ void k_ghost3(const DevPatch* __restrict__ PT, const int* __restrict__ patches,
                          const OverlapCopy* __restrict__ cps, const int2* __restrict__ ranges,
                          int ipass) {
+  after_previous();
   ghost3_patch(PT, patches[blockIdx.x], cps, ranges[blockIdx.x], ipass);
 }
 
@@ -457,6 +459,7 @@ __device__ __forceinline__ void filldown_item(const DevPatch* __restrict__ PT, c
 template <int D>
 __global__ void __launch_bounds__(BLOCK_THREADS)
     k_filldown(const DevPatch* __restrict__ PT, const Item* __restrict__ items) {
+  after_previous();
   filldown_item<D>(PT, items[blockIdx.x]);
 }
 

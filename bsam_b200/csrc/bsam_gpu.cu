@@ -312,20 +312,39 @@ void drain_events(bsam_gpu* h) {
 
 // ---- typed launches -----------------------------------------------------------
 
+// Launches a kernel that starts with after_previous(): its launch overlaps the
+// kernel before it, one to two microseconds of the five that a small level's
+// kernel takes.  Solves: 320 x 200 2.67 -> 2.55 ms, 512^2 mixed 4.8 -> 4.54, 96 x
+// 64 x 80 mixed 8.72 -> 8.47, 128^3 16.8 -> 16.5.
+template <class... P, class... A>
+void launch_after(bsam_gpu* h, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = h->stream;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, k, static_cast<P>(args)...);
+}
+
 template <class T, int D>
 void launch_relax_t(bsam_gpu* h, const LevelPlan& L, int color) {
-  k_relax<T, D><<<L.nfine, block_dim(), 0, h->stream>>>(h->d_patches, L.d_fine, color);
+  launch_after(h, k_relax<T, D>, L.nfine, block_dim(), 0, h->d_patches, L.d_fine, color);
 }
 
 // what: 0 = RestrictSolution, 2 = CoarseLoadingFunction, 1 = CorrectFine.
 template <class TC, class TP, int D>
 void launch_transfer_t(bsam_gpu* h, const LevelPlan& L, int what) {
   if (what == 0)
-    k_restrict<TC, TP, D><<<L.ncoarse, block_dim(), 0, h->stream>>>(h->d_patches, L.d_coarse);
+    launch_after(h, k_restrict<TC, TP, D>, L.ncoarse, block_dim(), 0, h->d_patches, L.d_coarse);
   else if (what == 2)
-    k_coarse_load<TC, TP, D><<<L.ncoarse, block_dim(), 0, h->stream>>>(h->d_patches, L.d_coarse);
+    launch_after(h, k_coarse_load<TC, TP, D>, L.ncoarse, block_dim(), 0, h->d_patches, L.d_coarse);
   else
-    k_correct<TC, TP, D><<<L.ncorr, block_dim(), 0, h->stream>>>(h->d_patches, L.d_corr);
+    launch_after(h, k_correct<TC, TP, D>, L.ncorr, block_dim(), 0, h->d_patches, L.d_corr);
 }
 
 // SetGhost(level, ipass) of a refined level (boundary.f90:58-89): coarse-fine
@@ -337,11 +356,11 @@ void amr_ghost(bsam_gpu* h, int level, int ipass) {
   const LevelPlan& L = plan(h, level);
   if (!L.amr) return;
   if (h->rp.ndims == 2) {
-    k_ghost2<<<L.nplist, 128, 0, h->stream>>>(h->d_patches, L.d_plist, L.d_ovl_by_dst,
-                                              L.d_ovl_range, ipass);
+    launch_after(h, k_ghost2, L.nplist, 128, 0, h->d_patches, L.d_plist, L.d_ovl_by_dst,
+                 L.d_ovl_range, ipass);
   } else {
-    k_ghost3<<<L.nplist, 256, 0, h->stream>>>(h->d_patches, L.d_plist, L.d_ovl_by_dst,
-                                              L.d_ovl_range, ipass);
+    launch_after(h, k_ghost3, L.nplist, 256, 0, h->d_patches, L.d_plist, L.d_ovl_by_dst,
+                 L.d_ovl_range, ipass);
   }
   ++h->stats.launches;
 }
@@ -354,7 +373,7 @@ void amr_ghost(bsam_gpu* h, int level, int ipass) {
 void snapshot(bsam_gpu* h, int level) {
   const LevelPlan& L = plan(h, level);
   if (!L.snap || L.nsnap == 0) return;
-  k_copy_spans<<<copy_spans_grid(L.snap_max, L.nsnap), 256, 0, h->stream>>>(L.d_snap);
+  launch_after(h, k_copy_spans, copy_spans_grid(L.snap_max, L.nsnap), 256, 0, L.d_snap);
   ++h->stats.launches;
 }
 
@@ -366,9 +385,9 @@ void filldown(bsam_gpu* h) {
   for (int level = h->finestlevel; level >= 1; --level) {
     const LevelPlan& L = plan(h, level);
     if (h->rp.ndims == 2)
-      k_filldown<2><<<L.ncoarse, block_dim(), 0, h->stream>>>(h->d_patches, L.d_coarse);
+      launch_after(h, k_filldown<2>, L.ncoarse, block_dim(), 0, h->d_patches, L.d_coarse);
     else
-      k_filldown<3><<<L.ncoarse, block_dim(), 0, h->stream>>>(h->d_patches, L.d_coarse);
+      launch_after(h, k_filldown<3>, L.ncoarse, block_dim(), 0, h->d_patches, L.d_coarse);
     ++h->stats.launches;
     amr_ghost(h, level - 1, 0);
   }
@@ -393,9 +412,9 @@ void launch_stage2_t(bsam_gpu* h, const LevelPlan& L, int dir) {
   const int upd = dir == 1 && P.master >= 0, nu = h->rp.nsmoothingpasses;
   auto tiles = [&](auto ty) {
     using S = Stage2<T, DELTA, decltype(ty)::value>;
-    k_stage2<T, DELTA, decltype(ty)::value>
-        <<<dim3(tx, (unsigned)(P.n[1] + S::TY - 1) / S::TY), S::THREADS, S::SMEM, h->stream>>>(
-            h->d_patches, p, dir, nu, upd);
+    launch_after(h, k_stage2<T, DELTA, decltype(ty)::value>,
+                 dim3(tx, (unsigned)(P.n[1] + S::TY - 1) / S::TY), S::THREADS, S::SMEM,
+                 h->d_patches, p, dir, nu, upd);
   };
   if (tx * ((unsigned)(P.n[1] + 15) / 16) >= 2 * 148) tiles(std::integral_constant<int, 16>{});
   else tiles(std::integral_constant<int, 8>{});
@@ -472,12 +491,14 @@ void launch_chain(bsam_gpu* h, const ChainLoop& loop) {
   cfg.blockDim = dim3(CHAIN_THREADS);
   cfg.dynamicSmemBytes = h->chain_smem;
   cfg.stream = h->stream;
-  cudaLaunchAttribute at{};
-  at.id = cudaLaunchAttributeClusterDimension;
-  at.val.clusterDim.x = (unsigned)h->chain_ctas;
-  at.val.clusterDim.y = at.val.clusterDim.z = 1;
-  cfg.attrs = &at;
-  cfg.numAttrs = 1;
+  cudaLaunchAttribute at[2]{};
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = (unsigned)h->chain_ctas;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 2;
   auto k = h->rp.ndims == 2 ? (h->mixed ? k_chain<2, true> : k_chain<2, false>)
                             : (h->mixed ? k_chain<3, true> : k_chain<3, false>);
   (void)cudaLaunchKernelEx(&cfg, k, (const DevPatch*)h->d_patches,
@@ -509,19 +530,16 @@ void launch_resid(bsam_gpu* h) {
   const unsigned g = (unsigned)(h->nmaster + TILE_Y - 1) / TILE_Y;
   if (!h->mixed) {
     if (nd == 2)
-      k_resid_norm<2><<<g, b, 0, h->stream>>>(
-          h->d_patches, h->d_master, h->d_partials, h->d_status, h->nmaster, h->denom,
-          h->rp.qerrortol);
+      launch_after(h, k_resid_norm<2>, g, b, 0, h->d_patches, h->d_master, h->d_partials,
+                   h->d_status, h->nmaster, h->denom, h->rp.qerrortol);
     else
-      k_resid_norm<3><<<g, b, 0, h->stream>>>(
-          h->d_patches, h->d_master, h->d_partials, h->d_status, h->nmaster, h->denom,
-          h->rp.qerrortol);
+      launch_after(h, k_resid_norm<3>, g, b, 0, h->d_patches, h->d_master, h->d_partials,
+                   h->d_status, h->nmaster, h->denom, h->rp.qerrortol);
   } else {
     const bool f32 = plan(h, h->finestlevel).prec == PREC_F32;
-#define DEFECT(TW, D)                                                                        \
-  k_defect<TW, D><<<g, b, 0, h->stream>>>(h->d_patches, h->d_master, h->d_partials, \
-                                                   h->d_status, h->nmaster, h->denom,        \
-                                                   h->rp.qerrortol)
+#define DEFECT(TW, D)                                                                     \
+  launch_after(h, k_defect<TW, D>, g, b, 0, h->d_patches, h->d_master, h->d_partials, \
+               h->d_status, h->nmaster, h->denom, h->rp.qerrortol)
     if (nd == 2) {
       if (f32) DEFECT(float, 2);
       else DEFECT(double, 2);
@@ -541,11 +559,11 @@ void launch_update(bsam_gpu* h) {
   const bool f32 = L.prec == PREC_F32;
   const dim3 b = block_dim();
   if (nd == 2) {
-    if (f32) k_update<float, 2><<<L.nfine, b, 0, h->stream>>>(h->d_patches, L.d_fine);
-    else k_update<double, 2><<<L.nfine, b, 0, h->stream>>>(h->d_patches, L.d_fine);
+    if (f32) launch_after(h, k_update<float, 2>, L.nfine, b, 0, h->d_patches, L.d_fine);
+    else launch_after(h, k_update<double, 2>, L.nfine, b, 0, h->d_patches, L.d_fine);
   } else {
-    if (f32) k_update<float, 3><<<L.nfine, b, 0, h->stream>>>(h->d_patches, L.d_fine);
-    else k_update<double, 3><<<L.nfine, b, 0, h->stream>>>(h->d_patches, L.d_fine);
+    if (f32) launch_after(h, k_update<float, 3>, L.nfine, b, 0, h->d_patches, L.d_fine);
+    else launch_after(h, k_update<double, 3>, L.nfine, b, 0, h->d_patches, L.d_fine);
   }
   ++h->stats.launches;
 }
@@ -584,8 +602,8 @@ int build_step_graph(bsam_gpu* h) {
     if (e == cudaSuccess) {
       const int64_t before = h->stats.launches;
       iteration(h);
-      k_mg_loop<<<1, 1, 0, h->stream>>>(h->d_status, h->d_trace, h->rp.maxvcycles,
-                                         h->rp.qerrortol, handle);
+      launch_after(h, k_mg_loop, 1, 1, 0, h->d_status, h->d_trace, h->rp.maxvcycles,
+                   h->rp.qerrortol, handle);
       h->graph_kernels_per_vcycle = (int)(h->stats.launches - before) + 1;
       h->stats.launches = before;
       cudaGraph_t captured = nullptr;
@@ -1764,9 +1782,9 @@ int bsam_gpu_restrict_level(bsam_gpu* h, int level) {
   CU(cudaSetDevice(h->device));
   const LevelPlan& L = plan(h, level);
   if (h->rp.ndims == 2)
-    k_filldown<2><<<L.ncoarse, block_dim(), 0, h->stream>>>(h->d_patches, L.d_coarse);
+    launch_after(h, k_filldown<2>, L.ncoarse, block_dim(), 0, h->d_patches, L.d_coarse);
   else
-    k_filldown<3><<<L.ncoarse, block_dim(), 0, h->stream>>>(h->d_patches, L.d_coarse);
+    launch_after(h, k_filldown<3>, L.ncoarse, block_dim(), 0, h->d_patches, L.d_coarse);
   ++h->stats.launches;
   amr_ghost(h, level - 1, 0);
   CU(cudaGetLastError());

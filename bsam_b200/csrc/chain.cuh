@@ -937,6 +937,7 @@ __device__ __forceinline__ void chain_store(const DevPatch& G, const ChainLevel&
 template <int D, bool MIXED>
 __global__ void __launch_bounds__(CHAIN_THREADS, 1)
     k_chain(const DevPatch* __restrict__ PT, const ChainPlan* __restrict__ plans, ChainLoop loop) {
+  after_previous();
   __shared__ ChainPlan PL;
   __shared__ ChainSlab slabs[CHAIN_MAX_LEVELS];
   __shared__ int again;

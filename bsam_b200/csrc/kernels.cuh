@@ -27,6 +27,15 @@ namespace bsam {
 
 template <class T> __device__ __forceinline__ T* fld(void* p) { return static_cast<T*>(p); }
 
+// Programmatic dependent launch: a kernel that starts with this may be launched
+// (launch_after, bsam_gpu.cu) while the one before it still runs; here it waits
+// until that one has completed and its results are visible, and lets the next
+// one be launched in its turn.
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // The entries of an n-long work list a CTA takes: runs of `chunk`
 // consecutive entries, run r going to CTA r mod gridDim.x (chunk 1 is the
 // plain grid-stride order).  A list holds each problem's tiles in a row, so
@@ -801,6 +810,7 @@ __device__ __forceinline__ void source_item(const DevPatch* __restrict__ PT, con
 template <class T, int D>
 __global__ void __launch_bounds__(BLOCK_THREADS)
     k_relax(const DevPatch* __restrict__ PT, const Item* __restrict__ items, int color) {
+  after_previous();
   relax_item<T, D>(PT, items[blockIdx.x], color);
 }
 
@@ -811,6 +821,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, D == 2 ? 5 : 4)
     k_resid_norm(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
                  double* __restrict__ partials, DevStatus* __restrict__ st, int nitems,
                  double denom, double tol) {
+  after_previous();
   const int b = blockIdx.x * TILE_Y + threadIdx.y;  // a tile per warp
   if (b < nitems) {
     const Item it = items[b];
@@ -830,18 +841,21 @@ __global__ void __launch_bounds__(BLOCK_THREADS, D == 2 ? 5 : 4)
 template <class TC, class TP, int D>
 __global__ void __launch_bounds__(BLOCK_THREADS)
     k_restrict(const DevPatch* __restrict__ PT, const Item* __restrict__ items) {
+  after_previous();
   restrict_item<TC, TP, D>(PT, items[blockIdx.x]);
 }
 
 template <class TC, class TP, int D>
 __global__ void __launch_bounds__(BLOCK_THREADS)
     k_coarse_load(const DevPatch* __restrict__ PT, const Item* __restrict__ items) {
+  after_previous();
   coarse_load_item<TC, TP, D>(PT, items[blockIdx.x]);
 }
 
 template <class TC, class TP, int D>
 __global__ void __launch_bounds__(BLOCK_THREADS)
     k_correct(const DevPatch* __restrict__ PT, const Item* __restrict__ items) {
+  after_previous();
   correct_item<TC, TP, D>(PT, items[blockIdx.x]);
 }
 
@@ -964,6 +978,7 @@ static __global__ void k_mg_begin(DevStatus* __restrict__ st) {
 // host reports it) or when a kernel recorded an error.
 static __global__ void k_mg_loop(DevStatus* __restrict__ st, double* __restrict__ trace, int maxv,
                           double tol, cudaGraphConditionalHandle handle) {
+  after_previous();
   const int it = st->iters + 1;
   st->iters = it;
   const double r = st->residual;

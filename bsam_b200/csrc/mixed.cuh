@@ -104,6 +104,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4)
     k_defect(const DevPatch* __restrict__ PT, const Item* __restrict__ items,
              double* __restrict__ partials, DevStatus* __restrict__ st, int nitems,
              double denom, double tol) {
+  after_previous();
   const int b = blockIdx.x * TILE_Y + threadIdx.y;  // a tile per warp
   if (b < nitems) {
     const Item it = items[b];
@@ -123,6 +124,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 4)
 template <class TW, int D>
 __global__ void __launch_bounds__(BLOCK_THREADS)
     k_update(const DevPatch* __restrict__ PT, const Item* __restrict__ items) {
+  after_previous();
   update_item<TW, D>(PT, items[blockIdx.x]);
 }
 

@@ -322,6 +322,7 @@ struct CopySpan {
 // are aligned (field allocations are, and have even lengths): CopyQToQold at
 // 128^3 (67 MB read and written) 77 -> 21 us.
 __global__ void __launch_bounds__(256) k_copy_spans(const CopySpan* __restrict__ spans) {
+  after_previous();
   const CopySpan s = spans[blockIdx.y];
   const int64_t step = (int64_t)gridDim.x * blockDim.x;
   int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x;

@@ -63,6 +63,7 @@ __device__ __forceinline__ void stage2_correction(const DevPatch& C, const DevPa
 template <class T, bool DELTA, int TY>
 __global__ void __launch_bounds__(256)
     k_stage2(const DevPatch* __restrict__ PT, int patch, int dir, int nu, int upd) {
+  after_previous();
   using S = Stage2<T, DELTA, TY>;
   using V = typename Stage2V<T>::V;
   extern __shared__ __align__(16) unsigned char stage2_raw[];
