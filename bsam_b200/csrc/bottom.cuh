@@ -2,7 +2,8 @@
 //
 // Below a few thousand cells a level is far too small to fill the GPU, and a
 // launch per colour pass and per transfer makes the coarse levels of a
-// V-cycle launch-latency bound.  The batch's kb_bottom (batch.cuh) runs
+// V-cycle launch-latency bound.  For chains that do not fit in shared memory
+// (chain.cuh) the batch's kb_bottom (batch.cuh) runs
 // AFASVcycle (afas:488-521) for a whole chain of small uniform levels -- from
 // the chain's top patch down to the coarsest level and back -- inside one CTA,
 // with __syncthreads between the phases the reference separates (every colour

@@ -13,13 +13,13 @@
 // A tick (one V-cycle of every running problem + its control) is captured
 // once into a graph whose WHILE node repeats ticks on the device; the graph
 // is captured again only when a list outgrows its capacity or a problem with
-// more grid-kernel depths arrives.
+// more grid-kernel depths, or a larger bottom chain, arrives.
 //
 // Records of one slot (local index): FP64 form 0 = root (level 0), l =
 // level -l; mixed form 0 = FP64 master, 1 = working twin of the root,
 // l + 1 = level -l.  Depth d of the V-cycle is level -d.  Depths whose
 // levels have more than bottom_cells cells run grid kernels ("top" depths);
-// the rest run inside the bottom kernel's chain, as in the single-problem
+// the rest run as a bottom chain (kb_chain, kb_bottom), as in the single-problem
 // engine with the same bottom_cells, and are FP64 in both forms.
 #include <cuda.h>
 #include <cudaTypedefs.h>
