@@ -43,8 +43,9 @@ __device__ __forceinline__ void after_previous() {
 // run's first tile come from L1 instead of a chain of L2 round trips; the
 // order in which a CTA visits tiles changes no result.  A list too short to
 // give every CTA a run is taken tile by tile (fit): in runs of two the coarse
-// levels' lists kept half as many CTAs busy (24 problems of 32^3 and 64^3 20.8
-// ms, tile by tile 19.4; but colour passes of the finest level 37 and 43 us).
+// levels' lists kept half as many CTAs busy.  The ticks of 24 problems of 32^3 and
+// 64^3: runs of two throughout 20.8 ms, single tiles throughout 19.4; later, other
+// kernels having become faster, single tiles 16.8 and by this rule 16.4.
 struct TileRuns {
   int chunk;
   __device__ __forceinline__ TileRuns fit(int n, int takers) const {
