@@ -104,11 +104,34 @@ struct ChainSlab {
 };
 
 // Rows [first, first + count) of CTA r of a level.
-__device__ __forceinline__ void chain_rows(const ChainLevel& L, int r, int& first, int& count) {
+__host__ __device__ __forceinline__ void chain_rows(const ChainLevel& L, int r, int& first, int& count) {
   const int per = L.ns % 2 ? 1 : 2;
   const int a = r * L.units / L.active, b = (r + 1) * L.units / L.active;
   first = a * per + 1;
   count = (b - a) * per;
+}
+
+// CTA `rank`'s part of a level; no rows (nr = 0) beyond the level's active CTAs.
+template <int D>
+__host__ __device__ __forceinline__ ChainSlab chain_slab(const ChainLevel& L, int rank) {
+  ChainSlab S{};
+  S.lo = 1;
+  S.lo_r = S.hi_r = -1;
+  if (rank >= L.active) return S;
+  chain_rows(L, rank, S.lo, S.nr);
+  const bool per = L.bc[2 * D - 2] == BC_PERIODIC;
+  if (L.active > 1 && (rank > 0 || per)) {
+    const int nb = rank > 0 ? rank - 1 : L.active - 1;
+    int first, count;
+    chain_rows(L, nb, first, count);
+    S.lo_r = nb;
+    S.lo_t = count + 1;
+  }
+  if (L.active > 1 && (rank + 1 < L.active || per)) {
+    S.hi_r = rank + 1 < L.active ? rank + 1 : 0;
+    S.hi_t = 0;
+  }
+  return S;
 }
 
 // The CTA that holds row k (1-based) of a level: the last one that starts at or
@@ -118,7 +141,8 @@ __device__ __forceinline__ int chain_owner(const ChainLevel& L, int k) {
   return (u * L.active - 1) / L.units;
 }
 
-template <int D> __device__ __forceinline__ int chain_idx(const ChainLevel& L, int i, int j, int t) {
+template <int D>
+__host__ __device__ __forceinline__ int chain_idx(const ChainLevel& L, int i, int j, int t) {
   return D == 2 ? i + t * L.sstr : i + j * L.pitch + t * L.sstr;
 }
 
@@ -188,8 +212,8 @@ template <class T> __device__ __forceinline__ T chain_map(int code, T v) {
   return code == BC_REFLECT ? T(2) + w : w;
 }
 
-__device__ __forceinline__ uint32_t chain_div(uint32_t x, uint32_t d, uint32_t m) {
-  return d == 1 ? x : __umulhi(x, m);
+__host__ __device__ __forceinline__ uint32_t chain_div(uint32_t x, uint32_t d, uint32_t m) {
+  return d == 1 ? x : (uint32_t)(((uint64_t)x * m) >> 32);
 }
 
 // A cell: its index, and per dimension and side the address of the cell that
@@ -201,14 +225,15 @@ template <class T, int D> struct ChainCell {
   T p, m, f0, f1, b;  // state, right-hand side, base (correction form)
 };
 
-template <class T> __device__ __forceinline__ uint32_t chain_byte(uint32_t field, int idx) {
+template <class T>
+__host__ __device__ __forceinline__ uint32_t chain_byte(uint32_t field, int idx) {
   return field + (uint32_t)idx * (uint32_t)sizeof(typename ChainV<T>::V);
 }
 
 // The neighbours of the cell at index X.c, coordinates (i, j), row slot t.
 template <class T, int D>
-__device__ __forceinline__ void chain_nb(const ChainLevel& L, const ChainSlab& S, int i, int j,
-                                         int t, ChainCell<T, D>& X) {
+__host__ __device__ __forceinline__ void chain_nb(const ChainLevel& L, const ChainSlab& S, int i,
+                                                  int j, int t, ChainCell<T, D>& X) {
   X.code = 0;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
@@ -232,8 +257,8 @@ __device__ __forceinline__ void chain_nb(const ChainLevel& L, const ChainSlab& S
 // next one (fed from the other end, of the other colour): all but the first
 // pass read those in place.
 template <class T, int D>
-__device__ __forceinline__ void chain_nb_raw(const ChainLevel& L, bool first,
-                                             ChainCell<T, D>& X) {
+__host__ __device__ __forceinline__ void chain_nb_raw(const ChainLevel& L, bool first,
+                                                      ChainCell<T, D>& X) {
   X.code = 0;
 #pragma unroll
   for (int d = 0; d < D; ++d) {
@@ -374,6 +399,7 @@ template <class T, int D> struct ChainPair {
   ChainCell<T, D> A, B;  // the cells of colours 0 and 1 (even and odd coordinate sums)
   int ic, jc, tc;        // coarse x, y (3D), and row of the slab in pairs (1-based)
   int t, j;              // row slot, y (3D)
+  int c;                 // index of the left-hand cell
   bool on, right;        // right: A is the right-hand cell
   ChainPush push;        // of the left-hand cell
   __device__ __forceinline__ uint32_t shift(bool a) const {  // of cell A (a) or B
@@ -381,11 +407,24 @@ template <class T, int D> struct ChainPair {
   }
 };
 
+// The pairs of a CTA's slab.
+template <int D>
+__host__ __device__ __forceinline__ int chain_pairs(const ChainLevel& L, const ChainSlab& S) {
+  return (int)(L.w * L.h) * (S.nr >> 1) << (D - 1);
+}
+
+// Does a CTA run a level's phases?  Every thread of one that does runs them (whole
+// warps, for the shuffles; threads without a pair of their own work on pair 0 and
+// store nothing).  A CTA without rows of the level (more CTAs than units) only
+// keeps the barriers: it has no pair 0, and the cell across a periodic face that
+// chain_nb would give it lies a whole level away, beyond its shared memory.
+__host__ __device__ __forceinline__ bool chain_runs(const ChainSlab& S) { return S.nr > 0; }
+
 template <class T, int D>
-__device__ __forceinline__ void chain_pair(const ChainLevel& L, const ChainSlab& S, int idx,
-                                           ChainPair<T, D>& R) {
+__host__ __device__ __forceinline__ void chain_pair(const ChainLevel& L, const ChainSlab& S,
+                                                    int idx, ChainPair<T, D>& R) {
   constexpr int SUB = D - 1;  // bits of the pair in its coarse cell
-  R.on = idx < (int)(L.w * L.h) * (S.nr >> 1) << SUB;
+  R.on = idx < chain_pairs<D>(L, S);
   const uint32_t sub = idx & ((1 << SUB) - 1), u = R.on ? (uint32_t)idx >> SUB : 0u;
   const uint32_t r = chain_div(u, L.w, L.mw);
   R.ic = (int)(u - r * L.w) + 1;
@@ -398,11 +437,11 @@ __device__ __forceinline__ void chain_pair(const ChainLevel& L, const ChainSlab&
   // Slabs start at odd rows, so slot and row have the same parity.
   R.right = (i0 + R.j + R.t) & 1;
   const int c0 = chain_idx<D>(L, i0, R.j, R.t);
+  R.c = c0;
   R.A.c = c0 + (R.right ? 1 : 0);
   R.B.c = c0 + (R.right ? 0 : 1);
   chain_nb<T, D>(L, S, i0 + (R.right ? 1 : 0), R.j, R.t, R.A);
   chain_nb<T, D>(L, S, i0 + (R.right ? 0 : 1), R.j, R.t, R.B);
-  R.push = chain_push<T>(L, S, c0, R.t);
 }
 
 // RestrictSolution and the restricted residual (the first half of
@@ -636,15 +675,17 @@ __device__ __forceinline__ void chain_visit_pairs(const ChainCtx& X, int l, bool
   R.on = false;
   auto load = [&](int idx) {
     chain_pair<T, D>(L, S, idx, R);
+    R.push = chain_push<T>(L, S, R.c, R.t);
     // Lanes without a pair work on pair 0's values and store nothing.
     chain_fetch<T, D, DELTA>(L, R.A);
     chain_fetch<T, D, DELTA>(L, R.B);
   };
-  const int total = ((int)(L.w * L.h) * (S.nr >> 1)) << (D - 1);
+  const int total = chain_pairs<D>(L, S);
+  const bool runs = !SLAB || chain_runs(S);  // uniform per CTA
   // One phase over the pairs of this thread (whole warps, for the shuffles).
   auto each = [&](auto body) {
     if constexpr (SINGLE) {
-      body();
+      if (runs) body();
     } else {
       for (int base = threadIdx.x & ~31; base < total; base += nt) {
         load(base + (threadIdx.x & 31));
@@ -652,7 +693,7 @@ __device__ __forceinline__ void chain_visit_pairs(const ChainCtx& X, int l, bool
       }
     }
   };
-  if (SINGLE) load(threadIdx.x);
+  if (SINGLE && runs) load(threadIdx.x);
   if (up) {
     each([&] {
       if (R.on) chain_up<T, TP, D, SLAB>(X, L, S, R, P);
@@ -955,25 +996,7 @@ __global__ void __launch_bounds__(CHAIN_THREADS, 1)
     L.qs += chain_base();
     L.bs += chain_base();
     if (threadIdx.x == 0) PL.rsum += chain_base();
-    ChainSlab S{};
-    S.lo = 1;
-    S.lo_r = S.hi_r = -1;
-    if (rank < L.active) {
-      chain_rows(L, rank, S.lo, S.nr);
-      const bool per = L.bc[2 * D - 2] == BC_PERIODIC;
-      if (L.active > 1 && (rank > 0 || per)) {
-        const int nb = rank > 0 ? rank - 1 : L.active - 1;
-        int first, count;
-        chain_rows(L, nb, first, count);
-        S.lo_r = nb;
-        S.lo_t = count + 1;
-      }
-      if (L.active > 1 && (rank + 1 < L.active || per)) {
-        S.hi_r = rank + 1 < L.active ? rank + 1 : 0;
-        S.hi_t = 0;
-      }
-    }
-    slabs[threadIdx.x] = S;
+    slabs[threadIdx.x] = chain_slab<D>(L, rank);
   }
   __syncthreads();
   const ChainCtx X{&PL, slabs, rank};

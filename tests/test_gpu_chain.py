@@ -93,3 +93,18 @@ def test_coarse_levels_are_readable(gpu_lib):
     for (qa, fa), (qb, fb) in zip(*out):
         assert np.array_equal(qa, qb)
         assert np.array_equal(fa, fb)
+
+
+# More CTAs in the cluster than the level has pairs of rows (planes), the last
+# dimension periodic: the CTAs without rows take no part in the level.
+@pytest.mark.parametrize("precision", [B.PREC_FP64, B.PREC_MIXED])
+@pytest.mark.parametrize("mx", [(110, 28), (98, 24), (44, 56), (126, 12), (10, 18, 24),
+                                (16, 24, 16), (22, 14, 12)])
+def test_clusters_with_ctas_without_rows(gpu_lib, mx, precision):
+    nd = len(mx)
+    prob = problem(mx, [1] * (2 * nd - 2) + [2, 2])
+    want = solve(prob, precision, -1)
+    got = solve(prob, precision, 0)
+    assert got[0] == want[0]
+    assert np.array_equal(got[1], want[1])
+    assert np.array_equal(got[2], want[2])
