@@ -213,7 +213,11 @@ template <class T> __device__ __forceinline__ T chain_map(int code, T v) {
 }
 
 __host__ __device__ __forceinline__ uint32_t chain_div(uint32_t x, uint32_t d, uint32_t m) {
+#ifdef __CUDA_ARCH__
+  return d == 1 ? x : __umulhi(x, m);
+#else
   return d == 1 ? x : (uint32_t)(((uint64_t)x * m) >> 32);
+#endif
 }
 
 // A cell: its index, and per dimension and side the address of the cell that
@@ -681,11 +685,10 @@ __device__ __forceinline__ void chain_visit_pairs(const ChainCtx& X, int l, bool
     chain_fetch<T, D, DELTA>(L, R.B);
   };
   const int total = chain_pairs<D>(L, S);
-  const bool runs = !SLAB || chain_runs(S);  // uniform per CTA
   // One phase over the pairs of this thread (whole warps, for the shuffles).
   auto each = [&](auto body) {
     if constexpr (SINGLE) {
-      if (runs) body();
+      body();
     } else {
       for (int base = threadIdx.x & ~31; base < total; base += nt) {
         load(base + (threadIdx.x & 31));
@@ -693,7 +696,7 @@ __device__ __forceinline__ void chain_visit_pairs(const ChainCtx& X, int l, bool
       }
     }
   };
-  if (SINGLE && runs) load(threadIdx.x);
+  if (SINGLE) load(threadIdx.x);
   if (up) {
     each([&] {
       if (R.on) chain_up<T, TP, D, SLAB>(X, L, S, R, P);
@@ -783,6 +786,12 @@ __device__ __noinline__ void chain_visit_t(const ChainCtx& X, int l, bool up, bo
   const ChainLevel L = X.PL->L[l];  // by value: its fields stay in registers
   const ChainSlab S = X.S[l];
   const bool last = l + 1 == X.PL->nlev;
+  if (SLAB && !chain_runs(S)) {
+    // The barriers of a visit: two a sweep, and where there is a coarser level one
+    // after the correction (up) or the restriction (down).
+    for (int b = 2 * X.PL->nu + (last ? 0 : 1); b > 0; --b) chain_cluster_sync();
+    return;
+  }
   const int cells = L.n[0] * (D == 3 ? L.n[1] : 1) * S.nr, work = last ? cells : cells >> 1;
   const ChainSync<SLAB> sync{min(max((work + 31) / 32, 1), (int)blockDim.x / 32)};
   if (!SLAB && (int)threadIdx.x >= 32 * sync.warps) {
