@@ -11,7 +11,7 @@
 // library instead of allocated storage.
 //
 // Scratch: g_noalloc_scratch below, a file-scope __device__ array.  Every GPU
-// that loads this library holds it (NOALLOC_SCRATCH_BYTES) until the process
+// that loads this library holds it (512 KiB) until the process
 // exits.  All calls share it, so calls whose kernels overlap on the GPU (two
 // host threads, or two streams without ordering between them) race on it and
 // give wrong results; order such calls on one stream.
@@ -19,6 +19,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "../../include/bsam_gpu.h"
 #include "bsam_types.h"
@@ -28,18 +29,14 @@ using namespace bsam;
 
 namespace {
 
-// Partial sums, one per CTA (at most one per tile of 64 x 4 x 1 cells), plus the
-// ticket of the last-block-done reduction in the trailing 256 bytes.
+// Partial sums, one per CTA (at most one per tile of 64 x 4 x 1 cells).  Nothing
+// in it is carried from one call to the next: a call whose kernels overlapped
+// another's spoils no later one.
 constexpr int NOALLOC_MAX_TILES = BSAM_NOALLOC_MAX_TILES;
-constexpr int NOALLOC_TAIL_DOUBLES = 32;
-constexpr size_t NOALLOC_SCRATCH_BYTES =
-    sizeof(double) * (NOALLOC_MAX_TILES + NOALLOC_TAIL_DOUBLES);
 
-static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_MAX_TILES +
-                                                          NOALLOC_TAIL_DOUBLES];
-static_assert(sizeof(g_noalloc_scratch) == NOALLOC_SCRATCH_BYTES &&
-                  NOALLOC_SCRATCH_BYTES <= 512 * 1024 + 256,
-              "the scratch array is meant to stay near 512 KiB");
+static __device__ __align__(256) double g_noalloc_scratch[NOALLOC_MAX_TILES];
+static_assert(sizeof(g_noalloc_scratch) <= 512 * 1024,
+              "the scratch array is meant to stay at 512 KiB");
 
 // Device address of g_noalloc_scratch per device.  In host code the symbol
 // name is only a host-side stand-in, never a device address, so the address
@@ -75,7 +72,8 @@ template <int D>
 __global__ void __launch_bounds__(32 * NORM_WARPS, NORM_CTAS_PER_SM)
     k_resid_norm_noalloc(DevPatch P, const double* __restrict__ fbase, int64_t fsy,
                          int64_t fsz, int64_t fcomp, int nseg, int nchunk, int rows,
-                         int64_t pieces, double* __restrict__ scratch, double denom, double* __restrict__ out) {
+                         int64_t pieces, double* __restrict__ scratch) {
+  next_may_launch();
   const int lane = threadIdx.x & 31;
   double acc = 0.0;
   for (int64_t w = (int64_t)blockIdx.x * NORM_WARPS + (threadIdx.x >> 5); w < pieces;
@@ -127,12 +125,42 @@ __global__ void __launch_bounds__(32 * NORM_WARPS, NORM_CTAS_PER_SM)
     if (i <= P.n[0]) acc += sum;
   }
   const double bs = block_sum(acc);
-  double total;
-  uint32_t* ticket = reinterpret_cast<uint32_t*>(scratch + NOALLOC_MAX_TILES);
-  if (last_block_total(bs, scratch, ticket, (int)gridDim.x, total)) {
+  if (threadIdx.x == 0) scratch[blockIdx.x] = bs;
+}
+
+// The sum of the partials, in index order by BLOCK_THREADS strided sums, and the
+// norm.  A launch of its own, which overlaps the one before it: a ticket that
+// the last CTA to finish recognises itself by would have to outlive the call or be
+// cleared by every one.
+__global__ void __launch_bounds__(BLOCK_THREADS)
+    k_norm_total(const double* scratch, int count, double denom, double* __restrict__ out) {
+  after_previous();
+  double s = 0.0;
+  for (int b = threadIdx.x; b < count; b += BLOCK_THREADS) s += __ldcg(scratch + b);
+  const double total = block_sum(s);
+  if (threadIdx.x == 0) {
     out[0] = sqrt(total / denom);
     out[1] = total;
   }
+}
+
+template <int D, class... A>
+cudaError_t launch_norm(unsigned ctas, cudaStream_t s, double* scratch, double denom, double* out,
+                        A... args) {
+  k_resid_norm_noalloc<D><<<ctas, 32 * NORM_WARPS, 0, s>>>(args..., scratch);
+  const cudaError_t e = cudaGetLastError();
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(1);
+  cfg.blockDim = dim3(BLOCK_THREADS);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  (void)cudaLaunchKernelEx(&cfg, k_norm_total, (const double*)scratch, (int)ctas, denom, out);
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -174,8 +202,6 @@ extern "C" int bsam_gpu_resid_norm_noalloc(int device, int ndims, const int32_t*
     P.tmp1 = dt / h2;
     P.tmp2 = eps * eps / h2;
     const double denom = (double)(2 * n[0] * n[1] * n[2]);
-    // The ticket starts at zero (static storage) and the last CTA of every
-    // launch sets it back; the partials are written before they are read.
     const int64_t fsy = n[0], fsz = n[0] * n[1], fcomp = n[0] * n[1] * n[2];
     const int64_t nseg = (n[0] + 31) / 32;
     // Rows per piece: 16 where that still gives every resident warp one, fewer
@@ -186,13 +212,14 @@ extern "C" int bsam_gpu_resid_norm_noalloc(int device, int ndims, const int32_t*
     const int64_t nchunk = (n[1] + rows - 1) / rows;
     const int64_t pieces = nseg * nchunk * n[2];
     const int64_t ctas = std::min<int64_t>(kCtas, (pieces + NORM_WARPS - 1) / NORM_WARPS);
-    if (ndims == 2)
-      k_resid_norm_noalloc<2><<<(unsigned)ctas, 32 * NORM_WARPS, 0, s>>>(
-          P, f, fsy, fsz, fcomp, (int)nseg, (int)nchunk, (int)rows, pieces, scratch, denom, out);
-    else
-      k_resid_norm_noalloc<3><<<(unsigned)ctas, 32 * NORM_WARPS, 0, s>>>(
-          P, f, fsy, fsz, fcomp, (int)nseg, (int)nchunk, (int)rows, pieces, scratch, denom, out);
-    if (cudaGetLastError() != cudaSuccess) rc = BSAM_ERR_CUDA;
+    auto launch = [&](auto dim) {
+      return launch_norm<decltype(dim)::value>((unsigned)ctas, s, scratch, denom, out, P, f, fsy,
+                                               fsz, fcomp, (int)nseg, (int)nchunk, (int)rows,
+                                               pieces);
+    };
+    const cudaError_t e = ndims == 2 ? launch(std::integral_constant<int, 2>{})
+                                     : launch(std::integral_constant<int, 3>{});
+    if (e != cudaSuccess) rc = BSAM_ERR_CUDA;
   }
   cudaSetDevice(prev);
   return rc;

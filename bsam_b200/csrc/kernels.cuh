@@ -31,9 +31,12 @@ template <class T> __device__ __forceinline__ T* fld(void* p) { return static_ca
 // (launch_after, bsam_gpu.cu) while the one before it still runs; here it waits
 // until that one has completed and its results are visible, and lets the next
 // one be launched in its turn.
+__device__ __forceinline__ void next_may_launch() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
 __device__ __forceinline__ void after_previous() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  next_may_launch();
 }
 
 // The entries of an n-long work list a CTA takes: runs of `chunk`

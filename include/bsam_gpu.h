@@ -280,7 +280,7 @@ const char* bsam_gpu_last_error(bsam_gpu* h);
  * of the process: after a cudaDeviceReset of the device it is stale, so do
  * not call this entry point on a device that was reset.  All calls share the
  * scratch: calls whose kernels overlap on the GPU race and give wrong
- * results. */
+ * results (those calls alone: nothing is carried over to later ones). */
 #define BSAM_NOALLOC_MAX_TILES 65536
 int bsam_gpu_resid_norm_noalloc(int device, int ndims, const int32_t* mx, double dx, double dt,
                                 double eps, double alpha, const double* q, const double* f,

@@ -36,3 +36,69 @@ def test_norm_of_ragged_patches(gpu_lib, oracle, mx):
         got = out.cpu().numpy()
         np.testing.assert_allclose(got[1], total, rtol=1e-12)
         np.testing.assert_allclose(got[0], np.sqrt(total / (2.0 * np.prod(mx))), rtol=1e-12)
+
+
+def norm_call(lib, mx, q, f, out, stream):
+    m = (ctypes.c_int32 * 3)(*(list(mx) + [1] * (3 - len(mx))))
+    import torch
+    return lib.bsam_gpu_resid_norm_noalloc(
+        torch.cuda.current_device(), len(mx), m, 1.0 / mx[0], 1e-4, 0.02, 1.0,
+        ctypes.c_void_p(q.data_ptr()), ctypes.c_void_p(f.data_ptr()),
+        ctypes.c_void_p(out.data_ptr()), ctypes.c_void_p(stream.cuda_stream))
+
+
+def fields(mx, seed):
+    import torch
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    ring = int(np.prod([m + 2 for m in mx]))
+    q = 0.5 + 0.1 * torch.randn(2 * ring, generator=g, dtype=torch.float64, device="cuda")
+    f = 0.01 * torch.randn(2 * int(np.prod(mx)), generator=g, dtype=torch.float64, device="cuda")
+    return q, f
+
+
+def test_overlapping_calls_spoil_no_later_one(gpu_lib):
+    """Calls that overlap share the scratch and may be wrong themselves; what they
+    leave in it must not reach a later call."""
+    import torch
+    sizes = [(64, 200), (500, 300)]
+    data = [fields(mx, k) for k, mx in enumerate(sizes)]
+    outs = [torch.zeros(2, dtype=torch.float64, device="cuda") for _ in sizes]
+    main = torch.cuda.current_stream()
+    want = []
+    for mx, (q, f), out in zip(sizes, data, outs):
+        assert norm_call(gpu_lib, mx, q, f, out, main) == 0
+        torch.cuda.synchronize()
+        want.append(out.cpu().numpy().copy())
+    streams = [torch.cuda.Stream() for _ in sizes]
+    for _ in range(50):
+        for _ in range(4):
+            for mx, (q, f), out, st in zip(sizes, data, outs, streams):
+                assert norm_call(gpu_lib, mx, q, f, out, st) == 0
+        torch.cuda.synchronize()
+        for mx, (q, f), out, w in zip(sizes, data, outs, want):
+            out.fill_(-1.0)
+            assert norm_call(gpu_lib, mx, q, f, out, main) == 0
+            torch.cuda.synchronize()
+            assert np.array_equal(out.cpu().numpy(), w)
+
+
+def test_captured_call_replays(gpu_lib):
+    import torch
+    mx = (500, 300)
+    q, f = fields(mx, 5)
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    assert norm_call(gpu_lib, mx, q, f, out, torch.cuda.current_stream()) == 0
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        assert norm_call(gpu_lib, mx, q, f, out, torch.cuda.current_stream()) == 0
+    for seed in (5, 6):
+        a, b = fields(mx, seed)
+        want = torch.zeros(2, dtype=torch.float64, device="cuda")
+        assert norm_call(gpu_lib, mx, a, b, want, torch.cuda.current_stream()) == 0
+        q.copy_(a)
+        f.copy_(b)
+        out.fill_(-1.0)
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want)
