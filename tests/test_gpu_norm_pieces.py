@@ -1,4 +1,4 @@
-"""bsam_gpu_resid_norm_noalloc at the edges of a warp's piece (32 columns, 4 to 16
+"""bsam_gpu_resid_norm_noalloc at the edges of a warp's piece (64 columns, 4 to 128
 rows) and of the grid, against the oracle's Operator.  Tolerance: the sums have
 at most 2e5 positive terms, each a few roundings off, added pairwise or in runs
 of at most a few hundred: 1e-12 relative is far above what that can reach."""
@@ -102,3 +102,36 @@ def test_captured_call_replays(gpu_lib):
         graph.replay()
         torch.cuda.synchronize()
         assert torch.equal(out, want)
+
+
+@pytest.mark.parametrize("mx", [(2, 2), (66, 6), (130, 34), (200, 72), (62, 1030), (512, 512),
+                                (2048, 1030), (6, 10, 4), (70, 10, 6), (128, 66, 34),
+                                (200, 96, 64)])
+def test_norm_is_the_solvers_bit_for_bit(gpu_lib, mx):
+    """The same number as the final residual of a solve of these fields."""
+    import torch
+
+    import bsam_b200 as B
+    from bsam_b200 import workloads as W
+    nd = len(mx)
+    rng = np.random.default_rng(sum(mx))
+    h = 1.0 / mx[0]
+    prob = W.Problem(ndims=nd, mx=tuple(mx) + (1,) * (3 - nd), eps=0.02, dt=1e-4, nsteps=1,
+                     qerrortol=1e-12, maxvcycles=2,
+                     xupper=tuple([n * h for n in mx] + [1.0] * (3 - nd)),
+                     c0=0.5 + 0.1 * rng.uniform(-1, 1, int(np.prod(mx))))
+    with B.Solver(prob) as s:
+        _, res, _ = s.step()
+        q, f, dx = s.get_q(), s.get_f(), s.patches[0].dx
+    qd = torch.from_numpy(q.ravel(order="F").copy()).cuda()
+    fd = torch.from_numpy(f.ravel(order="F").copy()).cuda()
+    out = torch.zeros(2, dtype=torch.float64, device="cuda")
+    m = (ctypes.c_int32 * 3)(*prob.mx)
+    rc = gpu_lib.bsam_gpu_resid_norm_noalloc(
+        torch.cuda.current_device(), nd, m, dx, prob.dt, prob.eps, prob.alpha,
+        ctypes.c_void_p(qd.data_ptr()), ctypes.c_void_p(fd.data_ptr()),
+        ctypes.c_void_p(out.data_ptr()),
+        ctypes.c_void_p(torch.cuda.current_stream().cuda_stream))
+    assert rc == 0
+    torch.cuda.synchronize()
+    assert out.cpu().numpy()[0] == res
