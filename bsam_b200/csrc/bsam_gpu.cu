@@ -24,7 +24,6 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
-#include <map>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -180,7 +179,7 @@ struct bsam_gpu {
   int nchains = 0, chain_ctas = 1;
   size_t chain_smem = 0;
   bool chain_loop = false;   // the chain is the whole solve: V-cycle loop in the kernel
-  int max_cluster = 1;       // CTAs of the largest cluster the device runs
+  int max_cluster = 0;       // CTAs of the largest cluster the device runs, 0: not asked yet
   double denom = 1.0;        // nrvars * cells of the finest level (ErrorAFAS)
   cudaGraphExec_t step_exec = nullptr;  // V-cycle loop graph (built lazily)
   int graph_kernels_per_vcycle = 0;
@@ -483,6 +482,12 @@ void transfer(bsam_gpu* h, int level, int what) {
   }
 }
 
+// The chain kernel of a handle's dimension and form.
+auto chain_kernel(const bsam_gpu* h) {
+  return h->rp.ndims == 2 ? (h->mixed ? k_chain<2, true> : k_chain<2, false>)
+                          : (h->mixed ? k_chain<3, true> : k_chain<3, false>);
+}
+
 // The chains below and including bottom_level (chain.cuh): one V-cycle, or
 // with loop.maxv > 0 MultigridIterations' whole loop.
 void launch_chain(bsam_gpu* h, const ChainLoop& loop) {
@@ -499,9 +504,7 @@ void launch_chain(bsam_gpu* h, const ChainLoop& loop) {
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 2;
-  auto k = h->rp.ndims == 2 ? (h->mixed ? k_chain<2, true> : k_chain<2, false>)
-                            : (h->mixed ? k_chain<3, true> : k_chain<3, false>);
-  (void)cudaLaunchKernelEx(&cfg, k, (const DevPatch*)h->d_patches,
+  (void)cudaLaunchKernelEx(&cfg, chain_kernel(h), (const DevPatch*)h->d_patches,
                            (const ChainPlan*)h->d_chains, loop);
   ++h->stats.launches;
 }
@@ -899,44 +902,39 @@ static void free_hierarchy(bsam_gpu* h) {
   h->have_hierarchy = false;
 }
 
-// Sets k_chain's attributes and returns the CTAs of the largest cluster of it
-// that the device can hold (16 need a GPC with 16 free SMs, 8 always fit;
-// negative: a CUDA error).  The attributes belong to the device's context and
-// the answer to the device, so both are settled once per device: the queries
-// take milliseconds.
-static int chain_cluster(int device) {
-  static std::mutex mutex;
-  static std::map<int, int> known;
-  std::lock_guard<std::mutex> lock(mutex);
-  const auto it = known.find(device);
-  if (it != known.end()) return it->second;
-  int most = CHAIN_MAX_CTAS;
-  auto one = [&](auto k) {
-    if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)CHAIN_SMEM_MAX) != cudaSuccess ||
-        cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
-      return false;
-    cudaLaunchConfig_t cfg{};
-    cfg.gridDim = dim3(CHAIN_MAX_CTAS);
-    cfg.blockDim = dim3(CHAIN_THREADS);
-    cfg.dynamicSmemBytes = CHAIN_SMEM_MAX;
-    cudaLaunchAttribute at{};
-    at.id = cudaLaunchAttributeClusterDimension;
-    at.val.clusterDim.x = CHAIN_MAX_CTAS;
-    at.val.clusterDim.y = at.val.clusterDim.z = 1;
-    cfg.attrs = &at;
-    cfg.numAttrs = 1;
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
-      cudaGetLastError();
-      most = 8;
-    }
-    return true;
-  };
-  if (!one(k_chain<2, false>) || !one(k_chain<2, true>) || !one(k_chain<3, false>) ||
-      !one(k_chain<3, true>))
+// Sets the attributes of the handle's chain kernel and returns the CTAs of the
+// largest cluster of it that the device can hold (16 need a GPC with 16 free SMs,
+// 8 always fit; negative: a CUDA error).  The attributes belong to the device's
+// context, which a reset replaces: every handle sets its own.  The answer is the
+// device's and is asked for once: the query takes milliseconds.
+static int chain_cluster(const bsam_gpu* h) {
+  constexpr int DEVICES = 64;
+  static std::atomic<int> known[DEVICES][4];
+  const auto k = chain_kernel(h);
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           (int)CHAIN_SMEM_MAX) != cudaSuccess ||
+      cudaFuncSetAttribute(k, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
     return -1;
-  known[device] = most;
+  const int form = (h->rp.ndims == 3 ? 2 : 0) + (h->mixed ? 1 : 0);
+  int most = h->device < DEVICES ? known[h->device][form].load() : 0;
+  if (most != 0) return most;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(CHAIN_MAX_CTAS);
+  cfg.blockDim = dim3(CHAIN_THREADS);
+  cfg.dynamicSmemBytes = CHAIN_SMEM_MAX;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = CHAIN_MAX_CTAS;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  int n = 0;
+  most = CHAIN_MAX_CTAS;
+  if (cudaOccupancyMaxActiveClusters(&n, k, &cfg) != cudaSuccess || n < 1) {
+    cudaGetLastError();
+    most = 8;
+  }
+  if (h->device < DEVICES) known[h->device][form].store(most);
   return most;
 }
 
@@ -1024,8 +1022,10 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
   int64_t bmax = dflt ? INT64_MAX : h->tuning.bottom_cells;
   if (dflt && h->tuning.fuse_smoother != 0)
     bmax = nd == 3 ? FUSED_BOTTOM_CELLS_3D : FUSED_BOTTOM_CELLS_2D;
-  if ((h->max_cluster = chain_cluster(h->device)) < 0)
+  if (h->max_cluster == 0 && (h->max_cluster = chain_cluster(h)) < 0) {
+    h->max_cluster = 0;
     return fail(h, BSAM_ERR_CUDA, "the chain kernel's attributes were rejected");
+  }
   h->bottom_level = -1000;
   h->chain_loop = false;
   std::vector<std::vector<int>> chains;  // per chain its patches, top first

@@ -69,7 +69,8 @@ int scratch_for_device(int device, double** out) {
 // Lane l holds columns l and l + 32, which keeps every load whole lines; the tree's
 // pairs (columns 2m, 2m + 1) then meet across neighbouring lanes, its lanes m and
 // m + 16 within one.  Bound by HBM latency: a tile's four rows of two columns
-// unrolled keep their loads in flight, for which a thread needs 128 registers (4096^2, 537 MB: 100 us = 5.3 TB/s with two CTAs per SM; 120 with three of 80
+// unrolled keep their loads in flight, for which a thread needs 128 registers (4096^2,
+// 537 MB: 100 us = 5.3 TB/s with two CTAs per SM; 120 with three of 80
 // registers or four of 64.  128^3 18.6 against 25, 256^3 120 against 252.  Warps of
 // 32 columns with sums in an order of their own took 113, 23 and 167.)
 constexpr int NORM_WARPS = 8;

@@ -108,3 +108,40 @@ def test_clusters_with_ctas_without_rows(gpu_lib, mx, precision):
     assert got[0] == want[0]
     assert np.array_equal(got[1], want[1])
     assert np.array_equal(got[2], want[2])
+
+
+RESET = """
+import ctypes, glob, os, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+import bsam_b200 as B
+from bsam_b200 import workloads as W
+import torch
+
+def solve(nd, precision):
+    prob = W.config1(nsteps=1, n=128) if nd == 2 else W.config3(nsteps=1, n=32)
+    with B.Solver(prob, precision=precision) as s:
+        return s.step(), s.get_q()
+
+forms = [(2, B.PREC_FP64), (2, B.PREC_MIXED), (3, B.PREC_FP64)]
+want = [solve(*f) for f in forms]
+names = glob.glob("/usr/local/cuda/lib64/libcudart.so*") + glob.glob(
+    os.path.join(os.path.dirname(torch.__file__), "..", "nvidia", "*", "lib", "libcudart.so*"))
+assert ctypes.CDLL(sorted(names)[0]).cudaDeviceReset() == 0
+for f, w in zip(forms, want):
+    got = solve(*f)
+    assert got[0] == w[0] and np.array_equal(got[1], w[1]), f
+print("equal after the reset")
+"""
+
+
+def test_handles_of_a_context_after_a_reset(gpu_lib):
+    """The chain kernel's attributes go with the context: a new handle after
+    cudaDeviceReset (of this process's own context) sets them anew."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", RESET, root], capture_output=True, text=True,
+                       timeout=300)
+    assert "equal after the reset" in r.stdout, r.stderr[-2000:]
