@@ -511,7 +511,9 @@ void launch_chain(bsam_gpu* h, const ChainLoop& loop) {
 
 // AFASVcycle (afas:488-521).
 void vcycle(bsam_gpu* h, int level) {
-  if (level == h->bottom_level) {
+  // A finest level in the chain is run as launches while its stages are timed (the
+  // same bits), and with it the levels below.
+  if (level == h->bottom_level && !(h->profiling && level == h->finestlevel)) {
     launch_chain(h, ChainLoop{});  // AFASVcycle(level) down to the coarsest level
     return;
   }
