@@ -24,6 +24,7 @@
 #include <cmath>
 #include <cstdio>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <string>
 #include <thread>
@@ -778,8 +779,8 @@ constexpr size_t kPieceBlock = 2 * kCopyThreads * kPieceBytes;  // the slots of 
 // the next copies, until the last handle is destroyed.
 struct PieceBlocks {
   std::mutex mutex;
-  std::vector<void*> idle;
-  int handles = 0;
+  void* idle[2] = {};
+  int nidle = 0, handles = 0;
   static PieceBlocks& get() {
     static PieceBlocks* p = new PieceBlocks;  // outlives every handle
     return *p;
@@ -787,11 +788,7 @@ struct PieceBlocks {
   void* take() {
     {
       std::lock_guard<std::mutex> lock(mutex);
-      if (!idle.empty()) {
-        void* p = idle.back();
-        idle.pop_back();
-        return p;
-      }
+      if (nidle > 0) return idle[--nidle];
     }
     void* p = nullptr;
     return cudaHostAlloc(&p, kPieceBlock, cudaHostAllocPortable) == cudaSuccess ? p : nullptr;
@@ -799,21 +796,26 @@ struct PieceBlocks {
   void give(void* p) {
     {
       std::lock_guard<std::mutex> lock(mutex);
-      if (handles > 0 && idle.size() < 2) {
-        idle.push_back(p);
+      if (handles > 0 && nidle < 2) {
+        idle[nidle++] = p;
         return;
       }
     }
     cudaFreeHost(p);
   }
   void count(int d) {
-    std::vector<void*> drop;
+    void* drop[2] = {};
     {
       std::lock_guard<std::mutex> lock(mutex);
       handles += d;
-      if (handles == 0) drop.swap(idle);
+      if (handles == 0)
+        while (nidle > 0) {
+          --nidle;
+          drop[nidle] = idle[nidle];
+        }
     }
-    for (void* p : drop) cudaFreeHost(p);
+    for (void* p : drop)
+      if (p) cudaFreeHost(p);
   }
 };
 
@@ -1603,7 +1605,14 @@ static int field_ptr(bsam_gpu* h, int patch, int field, int comp, double** ptr, 
   return BSAM_OK;
 }
 
-static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir) {
+// taken = false: no page-locked memory was to be had and nothing was done.
+static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir, bool& taken) {
+  taken = true;
+  auto none = [&] {
+    cudaGetLastError();
+    taken = false;
+    return BSAM_OK;
+  };
   const int64_t rows = 2 * task.rows;
   const size_t row_bytes = sizeof(double) * task.e0;
   auto launch = [&](double* packed, int64_t r0, int64_t r1) {
@@ -1616,7 +1625,7 @@ static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir) {
   };
   if (row_bytes * rows <= kBounceBytes) {
     double* pin = static_cast<double*>(pin_reserve(h, row_bytes * rows));
-    if (!pin) return fail(h, BSAM_ERR_NOMEM, "page-locked staging allocation failed");
+    if (!pin) return none();
     if (dir == 0) std::memcpy(pin, host, row_bytes * rows);
     CU(launch(pin, 0, rows));
     ++h->stats.launches;
@@ -1633,7 +1642,7 @@ static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir) {
   for (cudaEvent_t& e : h->slot_ev)
     if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
   char* pin = static_cast<char*>(PieceBlocks::get().take());
-  if (!pin) return fail(h, BSAM_ERR_NOMEM, "page-locked staging allocation failed");
+  if (!pin) return none();
   const int nt = (int)std::max(1u, std::min((unsigned)kCopyThreads,
                                             std::thread::hardware_concurrency()));
   std::atomic<int> failed{(int)cudaSuccess};
@@ -1670,9 +1679,15 @@ static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir) {
     }
     if (e != cudaSuccess) failed.store((int)e);
   };
+  // The shares of threads that cannot be had are done by this one.
   std::vector<std::thread> pool;
-  for (int t = 1; t < nt; ++t) pool.emplace_back(work, t);
+  int started = 1;
+  try {
+    for (; started < nt; ++started) pool.emplace_back(work, started);
+  } catch (const std::exception&) {
+  }
   work(0);
+  for (int t = started; t < nt; ++t) work(t);
   for (auto& t : pool) t.join();
   h->stats.launches += pieces;
   const cudaError_t done = cudaStreamSynchronize(h->stream);  // the block's next user may write it
@@ -1711,8 +1726,10 @@ static int copy_field(bsam_gpu* h, int patch, int field, double* host, int dir) 
         double* dev1;
         const int rc1 = field_ptr(h, patch, field, 1, &dev1, &interior);
         if (rc1) return fail(h, rc1, "field not held for this patch");
-        return copy_state(h, RowsTask{nullptr, {dev, dev1}, (int64_t)e1 * e2, P.sy, e0, 0}, host,
-                          dir);
+        bool taken;
+        const RowsTask task{nullptr, {dev, dev1}, (int64_t)e1 * e2, P.sy, e0, 0};
+        const int src = copy_state(h, task, host, dir, taken);
+        if (taken) return src;
       }
       if (dir == 0)
         CU(cudaMemcpy2DAsync(dev, P.sy * sizeof(double), hbase, e0 * sizeof(double),

@@ -37,3 +37,40 @@ def test_fields_come_back_as_put(gpu_lib, mx):
         s.put_q(b)
         s.get_q_into(out)
         assert np.array_equal(out, b)
+
+
+STARVED = """
+import ctypes, sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+import bsam_b200 as B
+from bsam_b200 import workloads as W
+
+mx = (1022, 1024)
+prob = W.Problem(ndims=2, mx=mx + (1,), eps=0.02, dt=1e-4, nsteps=1, qerrortol=1e-8,
+                 xupper=(1.0, mx[1] / mx[0], 1.0), c0=np.full(int(np.prod(mx)), 0.5))
+shape = tuple(m + 2 for m in mx) + (2,)
+a = np.asfortranarray(np.random.default_rng(1).standard_normal(shape))
+out = np.zeros(shape, order="F")
+s = B.Solver(prob)
+# Every thread started from here on wants a 64 TiB stack, which is refused.
+attr = ctypes.create_string_buffer(256)
+libc = ctypes.CDLL(None)
+assert libc.pthread_attr_init(attr) == 0
+assert libc.pthread_attr_setstacksize(attr, ctypes.c_size_t(1 << 46)) == 0
+assert libc.pthread_setattr_default_np(attr) == 0
+s.put_q(a)
+s.get_q_into(out)
+print("equal" if np.array_equal(a, out) else "different")
+"""
+
+
+def test_large_copies_without_threads(gpu_lib):
+    """Where no copy thread can be had, the calling thread does the work."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", STARVED, root], capture_output=True, text=True,
+                       timeout=300)
+    assert r.stdout.strip() == "equal", (r.returncode, r.stderr[-2000:])
