@@ -57,6 +57,8 @@ constexpr int FUSED_BOTTOM_CELLS_3D = 512;
 constexpr int64_t CHAIN_TOP_CELLS_2D = 128 * 128;
 constexpr int64_t CHAIN_TOP_CELLS_3D = 8192;
 
+constexpr int MAX_GRID_Y = 65535;
+
 struct LevelPlan {
   int level = 0;
   std::vector<int> patches;  // records the V-cycle runs on (ApplyOnLevel order)
@@ -372,9 +374,12 @@ void amr_ghost(bsam_gpu* h, int level, int ipass) {
 // nodes in a row).
 void snapshot(bsam_gpu* h, int level) {
   const LevelPlan& L = plan(h, level);
-  if (!L.snap || L.nsnap == 0) return;
-  launch_after(h, k_copy_spans, copy_spans_grid(L.snap_max, L.nsnap), 256, 0, L.d_snap);
-  ++h->stats.launches;
+  if (!L.snap) return;
+  for (int first = 0; first < L.nsnap; first += MAX_GRID_Y) {
+    const int n = std::min(MAX_GRID_Y, L.nsnap - first);
+    launch_after(h, k_copy_spans, copy_spans_grid(L.snap_max, n), 256, 0, L.d_snap + first);
+    ++h->stats.launches;
+  }
 }
 
 // FillDown(solutionfield) over the refined levels (afas:223-239): each
@@ -627,18 +632,20 @@ int build_step_graph(bsam_gpu* h) {
 }
 
 // SetBC on the FP64 state patches of the levels from `lo` to `hi` at and below
-// the root, in one launch (each reads and writes only itself).
+// the root, in one launch (each reads and writes only itself) per MAX_GRID_Y of them.
 void ghost_levels(bsam_gpu* h, int lo, int hi) {
   const int first = h->setbc_first[std::max(lo, h->minlevel) - h->minlevel];
   const int last = h->setbc_first[std::min(hi, 0) - h->minlevel + 1];
-  if (last <= first) return;
-  const dim3 g(setbc_blocks(h->rp.ndims, h->setbc_cells), (unsigned)(last - first));
-  const int* list = h->d_setbc + first;
-  if (h->rp.ndims == 2)
-    k_setbc_list<double, 2><<<g, SETBC_THREADS, 0, h->stream>>>(h->d_patches, list);
-  else
-    k_setbc_list<double, 3><<<g, SETBC_THREADS, 0, h->stream>>>(h->d_patches, list);
-  ++h->stats.launches;
+  for (int p = first; p < last; p += MAX_GRID_Y) {
+    const dim3 g(setbc_blocks(h->rp.ndims, h->setbc_cells),
+                 (unsigned)std::min(MAX_GRID_Y, last - p));
+    const int* list = h->d_setbc + p;
+    if (h->rp.ndims == 2)
+      k_setbc_list<double, 2><<<g, SETBC_THREADS, 0, h->stream>>>(h->d_patches, list);
+    else
+      k_setbc_list<double, 3><<<g, SETBC_THREADS, 0, h->stream>>>(h->d_patches, list);
+    ++h->stats.launches;
+  }
 }
 
 int face_rule(int ndims, int face, int code, int* rule) {
@@ -1070,6 +1077,9 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
       n = n == 0 ? 1 : 2;
     }
   for (char& n : alone) n = n == 1;
+  std::vector<char> has_child(npatch, 0);
+  for (int p = 0; p < npatch; ++p)
+    if (patches[p].parent >= 0 && patches[p].parent < npatch) has_child[patches[p].parent] = 1;
   const double eps2 = h->rp.eps * h->rp.eps;
   size_t total = 0;
   std::vector<size_t> offs(nrec);
@@ -1191,9 +1201,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     const int64_t vol = nd == 3 ? P.sz * (P.n[2] + 2) : P.sy * (P.n[1] + 2);
     h->field_elems[r] = roundup(lead + vol + 64, 256 / es);
     offs[r] = total;
-    bool parent_of_any = false;
-    if (in_vcycle)
-      for (int c = 0; c < npatch; ++c) parent_of_any |= patches[c].parent == p;
+    const bool parent_of_any = in_vcycle && has_child[p];
     const bool has_qold = !is_twin && d.level >= 0 && P.prec == PREC_F64 &&
                           (!h->mixed || d.level == finestlevel);
     nfields[r] = 2 /*q*/ + 2 /*f*/ + (has_qold ? 2 : 0) + (parent_of_any ? 2 : 0) +
@@ -1283,7 +1291,6 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     }
     h->setbc_first.push_back((int)setbc_list.size());
   }
-  if (setbc_list.size() > 65535) return fail(h, BSAM_ERR_ARG, "too many patches below the root");
   std::vector<CopySpan> snap_spans;
   std::vector<int> snap_first(h->levels.size() + 1, 0);
   for (size_t li = 0; li < h->levels.size(); ++li) {
@@ -1302,7 +1309,6 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
         L.snap_max = std::max(L.snap_max, h->field_elems[p]);
       }
     L.nsnap = (int)snap_spans.size() - snap_first[li];
-    if (L.nsnap > 65535) return fail(h, BSAM_ERR_ARG, "too many parent patches on a level");
   }
   // Parents of the twins are the masters' parents.
   for (int r = npatch; r < nrec; ++r) h->hp[r].parent = h->hp[rec_src[r]].parent;
