@@ -992,9 +992,10 @@ static bool find_chains(bsam_gpu* h, int npatch, const bsam_patch_desc* patches,
   return !plans.empty();
 }
 
-int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patches,
-                           int finestlevel) {
-  if (!h || npatch <= 0 || !patches) return BSAM_ERR_ARG;
+// stages2: 2D levels above the chain may run as stages (stage2.cuh), which need a
+// second state.
+static int set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patches, int finestlevel,
+                         bool stages2) {
   CU(cudaSetDevice(h->device));
   free_hierarchy(h);
   const int nd = h->rp.ndims;
@@ -1177,7 +1178,7 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     const bool fuse3 = h->tuning.fuse_smoother != 0 && nd == 3 && finestlevel == 0 && !periodic &&
                        !(P.delta && P.prec == PREC_F64) && P.n[0] >= fmin && P.n[1] >= fmin &&
                        P.n[2] >= fmin;
-    const bool fuse2 = nd == 2 && h->tuning.bottom_cells >= 0 && d.level <= 0 &&
+    const bool fuse2 = stages2 && nd == 2 && h->tuning.bottom_cells >= 0 && d.level <= 0 &&
                        h->rp.nsmoothingpasses <= 2 && alone[d.level - minlevel];
     P.fused = (fuse3 || fuse2) && in_vcycle && d.parent >= 0 && d.level > h->bottom_level ? 1 : 0;
     if (P.fused && nd == 3) {
@@ -1229,8 +1230,11 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
     // Under regridding the arena alternates with the spare: a quarter more
     // than this table needs lets the next tables of similar size reuse it.
     if (h->regridding) total += total / 4;
-    if (cudaMalloc(&h->d_arena, total) != cudaSuccess)
+    if (cudaMalloc(&h->d_arena, total) != cudaSuccess) {
+      cudaGetLastError();
+      h->d_arena = nullptr;
       return fail(h, BSAM_ERR_NOMEM, "arena allocation failed");
+    }
   }
   h->arena_bytes = total;
   CU(cudaMemsetAsync(h->d_arena, 0, total, h->stream));
@@ -1594,6 +1598,17 @@ int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patch
   CU(cudaStreamSynchronize(h->stream));
   h->have_hierarchy = true;
   return BSAM_OK;
+}
+
+int bsam_gpu_set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patches,
+                           int finestlevel) {
+  if (!h || npatch <= 0 || !patches) return BSAM_ERR_ARG;
+  const int rc = set_hierarchy(h, npatch, patches, finestlevel, true);
+  // Where the second states of the 2D stages do not fit beside the rest, every pass
+  // is a launch of its own (the same bits).
+  if (rc == BSAM_ERR_NOMEM && h->rp.ndims == 2)
+    return set_hierarchy(h, npatch, patches, finestlevel, false);
+  return rc;
 }
 
 static int field_ptr(bsam_gpu* h, int patch, int field, int comp, double** ptr, bool* interior) {

@@ -84,3 +84,46 @@ def test_first_sweep_reads_the_ghosts_as_given(gpu_lib, faces):
     assert out[0][:2] == out[1][:2]
     assert np.array_equal(out[0][2], out[1][2])
     assert np.array_equal(out[0][3], out[1][3])
+
+
+SHORT = """
+import sys
+import numpy as np
+sys.path.insert(0, sys.argv[1])
+import torch
+import bsam_b200 as B
+from bsam_b200 import workloads as W
+
+n = 4096
+rng = np.random.default_rng(1)
+prob = W.Problem(ndims=2, mx=(n, n, 1), eps=0.02, dt=1e-6, nsteps=1, qerrortol=1e-12,
+                 maxvcycles=1, c0=0.5 + 0.1 * rng.uniform(-1, 1, n * n))
+q0 = prob.q0()
+
+def solve():
+    with B.Solver(prob, q0=q0) as s:
+        return s.step(), s.get_q(), torch.cuda.mem_get_info()[0]
+
+before = torch.cuda.mem_get_info()[0]
+want = solve()
+# Six fields a level (state, right-hand side, and qold or the snapshot) and two more
+# for the second states, 4/3 of the root's in all: leave room for seven.
+field = (n + 2) * (n + 32) * 8
+spare = torch.cuda.mem_get_info()[0] - int(7 * 4 / 3 * field)
+hold = torch.empty(spare, dtype=torch.uint8, device="cuda")
+got = solve()
+assert got[0] == want[0] and np.array_equal(got[1], want[1])
+print("equal", before - want[2], got[2])
+"""
+
+
+def test_without_room_for_a_second_state(gpu_lib):
+    """A problem that fits the device only without the stages' second state runs as
+    launches, with the same result."""
+    import os
+    import subprocess
+    import sys
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    r = subprocess.run([sys.executable, "-c", SHORT, root], capture_output=True, text=True,
+                       timeout=300)
+    assert r.stdout.startswith("equal"), (r.returncode, r.stdout, r.stderr[-2000:])
