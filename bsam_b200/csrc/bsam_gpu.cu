@@ -55,7 +55,7 @@ constexpr int FUSED_BOTTOM_CELLS_2D = 1024;
 constexpr int FUSED_BOTTOM_CELLS_3D = 512;
 // Largest level of the bottom chain where other levels run above it.
 constexpr int64_t CHAIN_TOP_CELLS_2D = 128 * 128;
-constexpr int64_t CHAIN_TOP_CELLS_3D = 8192;
+constexpr int64_t CHAIN_TOP_CELLS_3D = 16384;
 
 constexpr int MAX_GRID_Y = 65535;
 
@@ -1023,13 +1023,16 @@ static int set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patches
   // there.  A whole FP64 problem that fits does: its V-cycle loop runs in the
   // one launch (192^2 V-cycle 70 us, against 85 with its finest level as
   // stages).  Below other levels a chain's top level has 16 SMs against all of
-  // them: in 2D a level of 128^2 still costs less in the chain (256^2 FP64 97
-  // against 102 us a V-cycle, 256^2 mixed 107 against 113) and one of 192^2 or
-  // 256^2 less as stages (512^2 mixed 140 against 160 us); in 3D a level of
-  // 16^3 (64^3 FP64 181 against 197 us) or 24 x 16 x 20 (96 x 64 x 80 mixed 218
-  // against 235) costs less in the chain and one of 32^3 less as launches (64^3
-  // 181 against 191, 128^3 491 against 505).  A caller's bottom_cells stands as
-  // given.
+  // them.  In 2D a level of 128^2 still costs less in the chain (256^2 FP64 97
+  // against 102 us a V-cycle, 256^2 mixed 107 against 113), one of 144^2, 160 x 128
+  // or 160^2 the same or more (a step of four V-cycles of 288^2 FP64 417 against 408
+  // us, of 320 x 256 mixed 487 against 472) and one of 192^2 or 256^2 more (512^2
+  // mixed 140 against 160 us a V-cycle).  In 3D a level of 20 x 20 x 24, 20 x 24 x 28
+  // or 24^3 costs less in the chain (a step of 40 x 40 x 48 FP64 505 against 604 us,
+  // of 40 x 48 x 56 545 against 628, of 48^3 605 against 656; mixed 556 against 640,
+  // 580 against 645, 651 against 695), one of 28^3 about the same (56^3 FP64 643
+  // against 663, mixed 690 against 692) and one of 32^3 more (64^3 FP64 191 against
+  // 181 us a V-cycle, 128^3 505 against 491).  A caller's bottom_cells stands as given.
   const int64_t chain_top = nd == 3 ? CHAIN_TOP_CELLS_3D : CHAIN_TOP_CELLS_2D;
   int64_t bmax = dflt ? INT64_MAX : h->tuning.bottom_cells;
   if (dflt && h->tuning.fuse_smoother != 0)

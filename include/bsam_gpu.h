@@ -88,7 +88,7 @@ int bsam_gpu_create(bsam_gpu** h, int device, const bsam_run_params* p);
  *                  the V-cycle in one launch (a thread-block cluster, the
  *                  levels in its shared memory) as far as they fit there;
  *                  0 = default (those that cost less there: a whole problem
- *                  that fits, else levels of at most 128^2 cells, 8192 in 3D),
+ *                  that fits, else levels of at most 128^2 cells, 16384 in 3D),
  *                  -1 = never, and every level one launch per pass.  In the
  *                  mixed form levels of at most bottom_cells are FP64; under
  *                  the default and with -1, levels of at most 4096 cells are

@@ -110,6 +110,18 @@ def test_clusters_with_ctas_without_rows(gpu_lib, mx, precision):
     assert np.array_equal(got[2], want[2])
 
 
+@pytest.mark.parametrize("precision", [B.PREC_FP64, B.PREC_MIXED])
+@pytest.mark.parametrize("mx", [(256, 256), (40, 40, 48), (40, 48, 56), (48, 48, 48), (64, 32, 64)])
+def test_chains_of_the_largest_tops(gpu_lib, mx, precision):
+    """Levels just inside the size to which the chain reaches below other levels."""
+    prob = problem(mx, [10] * (2 * len(mx)))
+    want = solve(prob, precision, -1)
+    got = solve(prob, precision, 0)
+    assert got[0] == want[0]
+    assert np.array_equal(got[1], want[1])
+    assert np.array_equal(got[2], want[2])
+
+
 RESET = """
 import ctypes, glob, os, sys
 import numpy as np
