@@ -48,13 +48,6 @@ struct SlotCfg {
   double tol;
 };
 
-// The streaming kernels over tile lists are bound by memory latency.  For the
-// FP64 defect, the FP64 update and the 2D correction a register cap of 48
-// (ten 128-thread CTAs per SM) puts more loads in flight and measured 11-17 %
-// faster; restriction and coarse load measured slower under that cap (the
-// coarse load takes a cap of 64 instead).
-constexpr int BATCH_LATENCY_MIN_BLOCKS = 10;
-
 // Device-owned per-slot state (the host writes it only at admission).
 struct SlotState {
   int32_t phase, step, iters, vcycles;
@@ -385,7 +378,7 @@ __device__ __forceinline__ double seeded_c(const DevPatch& P, uint64_t seed, dou
   return cbar + amp * seeded_u(seed, idx);
 }
 
-// Interior of the state record `rec`: c and mu (ghosts by a k_setbc launch).
+// Interior of the state record `rec`: c and mu (ghosts by k_setbc_list).
 template <int D>
 __device__ __forceinline__ void init_seeded_range(const DevPatch& P, uint64_t seed, double cbar,
                                                   double amp, double k2, int64_t g0,

@@ -154,7 +154,7 @@ struct bsam_batch {
   cudaStream_t stream = nullptr;
   bsam_batch_params bp{};
   bool mixed = false;
-  int nsm = 148;
+  int nsm = B200_SMS;
   bsam_batch_tuning tuning{};
   // pool
   char* d_pool = nullptr;
@@ -573,7 +573,6 @@ int plan_slot(bsam_batch* b, const bsam_batch_problem* pr, int rec0, char* base,
   return BSAM_OK;
 }
 
-// Appends a slot's tiles to the lists and records its master range.
 // Does a bottom chain of these extents, top first, fit in a CTA's shared memory
 // (chain.cuh)?  Keeps the largest size so far.
 bool chain_fits(bsam_batch* b, const std::vector<std::array<int, 3>>& n, bool delta) {
@@ -588,6 +587,7 @@ bool chain_fits(bsam_batch* b, const std::vector<std::array<int, 3>>& n, bool de
   return true;
 }
 
+// Appends a slot's tiles to the lists and records its master range.
 void append_items(bsam_batch* b, int s) {
   SlotPlan& S = b->slots[s];
   const int nd = b->bp.ndims;

@@ -421,7 +421,8 @@ void launch_stage2_t(bsam_gpu* h, const LevelPlan& L, int dir) {
                  dim3(tx, (unsigned)(P.n[1] + S::TY - 1) / S::TY), S::THREADS, S::SMEM,
                  h->d_patches, p, dir, nu, upd);
   };
-  if (tx * ((unsigned)(P.n[1] + 15) / 16) >= 2 * 148) tiles(std::integral_constant<int, 16>{});
+  if (tx * ((unsigned)(P.n[1] + 15) / 16) >= 2 * B200_SMS)
+    tiles(std::integral_constant<int, 16>{});
   else tiles(std::integral_constant<int, 8>{});
   ++h->stats.launches;
 }
@@ -1191,7 +1192,7 @@ static int set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patches
       int chunk = h->tuning.chunk;
       if (chunk <= 0) {
         // About one CTA per SM, chunks of at least 16 planes.
-        const int nchunk = std::max(1, std::min(148 / std::max(tiles, 1), P.n[2] / 16));
+        const int nchunk = std::max(1, std::min(B200_SMS / std::max(tiles, 1), P.n[2] / 16));
         chunk = (P.n[2] + nchunk - 1) / nchunk;
       }
       P.zchunk = std::max(1, std::min(chunk, P.n[2]));

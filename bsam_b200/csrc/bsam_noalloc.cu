@@ -314,7 +314,7 @@ extern "C" int bsam_gpu_resid_norm_noalloc(int device, int ndims, const int32_t*
     const int64_t nseg = tiles_x;
     // Rows per piece, whole tiles: those for which the warps, each at its share of
     // the pieces, take the fewest rows (the row above a piece is loaded again).
-    const int64_t kCtas = 148 * NORM_CTAS_PER_SM;
+    const int64_t kCtas = B200_SMS * NORM_CTAS_PER_SM;
     int64_t rows = TILE_Y, least = INT64_MAX;
     for (int64_t r = TILE_Y; r <= 32 * TILE_Y; r += TILE_Y) {
       const int64_t all = nseg * ((n[1] + r - 1) / r) * n[2];

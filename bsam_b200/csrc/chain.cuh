@@ -454,9 +454,8 @@ __host__ __device__ __forceinline__ void chain_pair(const ChainLevel& L, const C
 // and the residual in f.  Sums in the reference's order of the children (x
 // fastest, from the high end).  Every lane of the warp calls it.
 template <class T, class TP, int D, bool DELTA>
-__device__ __forceinline__ void chain_down(const ChainCtx& X, const ChainLevel& L,
-                                           const ChainSlab& S, const ChainPair<T, D>& R,
-                                           const ChainLevel& P) {
+__device__ __forceinline__ void chain_down(const ChainLevel& L, const ChainSlab& S,
+                                           const ChainPair<T, D>& R, const ChainLevel& P) {
   constexpr unsigned FULL = 0xffffffffu;
   constexpr int NP = 1 << (D - 1);  // pairs of a coarse cell
   T rA0 = T(0), rA1 = T(0), rB0 = T(0), rB1 = T(0);
@@ -575,9 +574,8 @@ __device__ __forceinline__ void chain_down(const ChainCtx& X, const ChainLevel& 
 // cell takes 3/4 of its own coarse cell (near) and 1/4 of the next one on its
 // side (far) per dimension, x first: lin_x's sums, whose two terms commute.
 template <class T, class TP, int D, bool SLAB>
-__device__ __forceinline__ void chain_up(const ChainCtx& X, const ChainLevel& L,
-                                         const ChainSlab& S, ChainPair<T, D>& R,
-                                         const ChainLevel& P) {
+__device__ __forceinline__ void chain_up(const ChainLevel& L, const ChainSlab& S,
+                                         ChainPair<T, D>& R, const ChainLevel& P) {
   const int kc = (S.lo - 1) / 2 + R.tc;
   const int own = P.active == 1 ? 0 : chain_owner(P, kc);
   int first = 1, count = P.ns;
@@ -699,7 +697,7 @@ __device__ __forceinline__ void chain_visit_pairs(const ChainCtx& X, int l, bool
   if (SINGLE) load(threadIdx.x);
   if (up) {
     each([&] {
-      if (R.on) chain_up<T, TP, D, SLAB>(X, L, S, R, P);
+      if (R.on) chain_up<T, TP, D, SLAB>(L, S, R, P);
     });
     sync();
   } else if (l > 0) {
@@ -728,7 +726,7 @@ __device__ __forceinline__ void chain_visit_pairs(const ChainCtx& X, int l, bool
     sync();
   }
   if (!up) {
-    each([&] { chain_down<T, TP, D, DELTA>(X, L, S, R, P); });
+    each([&] { chain_down<T, TP, D, DELTA>(L, S, R, P); });
     sync();
   }
 }
@@ -844,8 +842,8 @@ __device__ __forceinline__ void chain_vcycle(const ChainCtx& X, bool raw) {
   for (int l = min(ns, nl - 1) - 1; l >= 0; --l) chain_visit<D, MIXED>(X, l, true, false);
 }
 
-// ErrorAFAS of the top level (FP64), summed in the order of resid_item,
-// block_sum and last_block_total: per tile of 64 x TILE_Y cells a shuffle
+// ErrorAFAS of the top level (FP64), summed in the order of resid_rows
+// and last_block_sum: per tile of 64 x TILE_Y cells a shuffle
 // tree per row, the rows in order; the tiles by 128 strided sums and the same
 // tree.  Valid in thread 0 of CTA 0.
 template <int D>

@@ -1,13 +1,12 @@
 // defect2.cuh -- the mixed form's FP64 defect of 2D masters, tiles staged by TMA.
 //
-// defect_item (mixed.cuh) reads the master's q with a 5-point stencil and f
-// straight from global memory, two cells per thread; at a few hundred cells
-// per tile those loads stall on memory latency (about 40 % of HBM bandwidth
-// measured).  Here one thread issues bulk tensor copies of the tile's q
+// The master's q with its 5-point stencil and f, read straight from global memory
+// with two cells per thread, stalled on memory latency at a few hundred cells per
+// tile (about 40 % of HBM bandwidth measured).  Here one thread issues bulk tensor copies of the tile's q
 // (both components, one-cell halo) and f into shared memory, and the CTA
-// computes from there.  Tiles, the thread-to-cell mapping, every expression
-// and the block reduction are those of defect_item, so each tile's partial
-// sum -- and so the residual -- is bit for bit the same.
+// computes from there.  Tiles, every expression and the order of the sums are
+// those of defect_rows (mixed.cuh), so each tile's partial sum -- and so the
+// residual -- is bit for bit the same.
 #pragma once
 #include "fused2.cuh"
 #include "mixed.cuh"
@@ -123,7 +122,7 @@ __global__ void __launch_bounds__(BLOCK_THREADS, 8)
       mw_patch = it.patch;
     }
     const int i0 = it.tx * F::TX + 1, j0 = it.ty * F::TY + 1;
-    // defect_item's cells of this thread, from the staged tile.
+    // This thread's two cells, from the staged tile.
     const int j = j0 + threadIdx.y;
     const int ic0 = (it.tx * 32 + threadIdx.x) * 2 + 1;
     double acc = 0.0;

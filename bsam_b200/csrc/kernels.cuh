@@ -25,6 +25,9 @@
 
 namespace bsam {
 
+// SMs of a B200: sizes of grids and shares of work; no result depends on it.
+constexpr int B200_SMS = 148;
+
 template <class T> __device__ __forceinline__ T* fld(void* p) { return static_cast<T*>(p); }
 
 // Programmatic dependent launch: a kernel that starts with this may be launched
@@ -298,19 +301,6 @@ __device__ __forceinline__ void operator_with(const DevPatch& P, const Problem::
     Problem::OperatorCell<T, D, true>(s, T(P.tmp1), T(P.tmp2), T(P.alpha), o0, o1, base);
   else
     Problem::OperatorCell<T, D>(s, T(P.tmp1), T(P.tmp2), T(P.alpha), o0, o1);
-}
-
-// Residual rf = f - Operator(q) at one cell (afas:799-840).
-template <class T, int D>
-__device__ __forceinline__ void residual_cell(const DevPatch& P, const T* q0, const T* q1,
-                                              const T* f0, const T* f1, int64_t c, T& r0,
-                                              T& r1) {
-  Problem::Stencil<T, D> s;
-  load_stencil<T, D>(P, q0, q1, c, s);
-  T o0, o1;
-  operator_at<T, D>(P, s, c, o0, o1);
-  r0 = f0[c] - o0;
-  r1 = f1[c] - o1;
 }
 
 // RestrictSolution (afas:600-644) of the coarse cell (ic,jc,kc) of child C

@@ -347,7 +347,7 @@ __global__ void __launch_bounds__(256) k_copy_spans(const CopySpan* __restrict__
 // The grid of k_copy_spans for nspans spans of at most `longest` elements: a
 // thread per four 16-byte accesses, at most 16 CTAs per SM in all.
 inline dim3 copy_spans_grid(int64_t longest, int64_t nspans) {
-  const int64_t want = (longest + 2047) / 2048, most = std::max<int64_t>(1, 16 * 148 / nspans);
+  const int64_t want = (longest + 2047) / 2048, most = std::max<int64_t>(1, 16 * B200_SMS / nspans);
   return dim3((unsigned)std::max<int64_t>(1, std::min(want, most)), (unsigned)nspans);
 }
 
