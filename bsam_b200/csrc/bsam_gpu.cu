@@ -1643,7 +1643,8 @@ static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir, bool& t
   auto launch = [&](double* packed, int64_t r0, int64_t r1) {
     RowsTask t = task;
     t.packed = packed - r0 * task.e0;  // so that row r0 lies at `packed`
-    const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((r1 - r0 + 7) / 8, 592));
+    const int64_t warps = (r1 - r0) * ((task.e0 + ROW_PART - 1) / ROW_PART);
+    const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((warps + 7) / 8, 592));
     if (dir == 0) k_rows<true><<<g, 256, 0, h->stream>>>(t, r0, r1);
     else k_rows<false><<<g, 256, 0, h->stream>>>(t, r0, r1);
     return cudaGetLastError();

@@ -39,6 +39,21 @@ def test_fields_come_back_as_put(gpu_lib, mx):
         assert np.array_equal(out, b)
 
 
+@pytest.mark.parametrize("mx", [(510, 8), (512, 1100), (1030, 1024), (2046, 300), (5000, 220),
+                                (4094, 2)])
+def test_long_rows(gpu_lib, mx):
+    """Rows of several parts, a warp each, on every copy path."""
+    rng = np.random.default_rng(sum(mx))
+    prob = W.Problem(ndims=2, mx=mx + (1,), eps=0.02, dt=1e-4, nsteps=1, qerrortol=1e-8,
+                     xupper=(1.0, mx[1] / mx[0], 1.0), c0=np.full(int(np.prod(mx)), 0.5))
+    a = np.asfortranarray(rng.standard_normal(tuple(m + 2 for m in mx) + (2,)))
+    out = np.zeros_like(a, order="F")
+    with B.Solver(prob) as s:
+        s.put_q(a)
+        s.get_q_into(out)
+    assert np.array_equal(out, a)
+
+
 STARVED = """
 import ctypes, sys
 import numpy as np
