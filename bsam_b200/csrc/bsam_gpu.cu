@@ -134,7 +134,9 @@ struct bsam_gpu {
   void* h_pin = nullptr;
   size_t pin_cap = 0;
   bool pin_busy = false;       // queued work still reads it (a put_field)
-  cudaEvent_t slot_ev[8] = {};  // put / get of large fields: a piece's slot is free / full
+  // put / get of large fields: a piece's slot is free / full; streams of host threads.
+  cudaEvent_t slot_ev[8] = {};
+  cudaStream_t copy_streams[3] = {};
   bool attrs_set = false;      // the fused kernels' shared-memory attributes
   uint8_t* d_flags = nullptr;  // bsam_gpu_errflags_level's device flags
   int32_t* d_sat = nullptr;    // bsam_gpu_tag_level's summed-area tables
@@ -766,64 +768,77 @@ int engine_device(bsam_gpu* h) { return h ? h->device : -1; }
 namespace {
 
 // put_field / get_field of q or qold (both components, ghost ring included)
-// between the caller's pageable array and the pitched fields, through
-// page-locked memory: a kernel spreads the rows from it, or packs them into it,
-// over the bus; a host copy does the rest.  For small fields, in the bounce
-// buffer, that is one launch instead of two staged pitched copies (a 16 KB
-// field: put 28 -> 12 us, get 27 -> 19).  Large fields go in pieces that a few
-// host threads copy side by side, each through two slots of its own, so that
-// host copies and the bus overlap (128^3, 35 MB: put 3.9 -> 1.2 ms, get 1.9 ->
-// 1.5).  Between the two limits the driver's pitched copies are as good (512^2,
-// 4 MB: 0.30 ms up and 0.28 down, 0.24 and 0.27 in pieces) and need no
-// page-locked memory, which costs 1 ms per MB to allocate.
+// between the caller's pageable array and the pitched fields, through page-locked
+// memory: a kernel spreads the rows from it, or packs them into it, over the bus; a
+// host copy does the rest.  For small fields, in the bounce buffer, that is one
+// launch instead of two staged pitched copies (a 16 KB field: put 28 -> 12 us, get
+// 27 -> 19).  Large fields go in pieces that a few host threads copy side by side,
+// each through two slots and on a stream of its own, so that host copies, launches
+// and the bus overlap.  Between the two limits the driver's pitched copies are as
+// good and need no page-locked memory, which costs 1 to 2 ms per MB to allocate:
+// hence as little of it as keeps the bus busy.  Against the driver's copies, in ms
+// (put, get, and a whole one-shot solve: create, a step, get, destroy): 96 x 64 x 80
+// (8.3 MB) 1.4 -> 0.55, 0.7 -> 0.65, 8.1 -> 7.3; 128^3 (35 MB) 4.0 -> 1.7, 1.8 to 2.6
+// -> 1.7, 14 -> 14; 192^3 13 -> 5.1, 5.8 to 7.6 -> 5.1, 33 -> 27.  Long rows suit the
+// driver: 1024 x 512 (8.4 MB) 0.54 -> 0.64, 0.70 -> 0.67; 2048^2 (67 MB) 6.0 -> 3.0,
+// 3.3 to 3.9 -> 3.0.
 constexpr size_t kBounceBytes = (size_t)128 << 10;
-constexpr size_t kThreadedBytes = (size_t)8 << 20;
-constexpr size_t kPieceBytes = (size_t)512 << 10;
 constexpr int kCopyThreads = 4;
-constexpr size_t kPieceBlock = 2 * kCopyThreads * kPieceBytes;  // the slots of one copy
+
+// Bytes of a slot for a field of `bytes` in rows of `row`, 0: not in pieces.
+size_t piece_bytes(size_t bytes, size_t row) {
+  const size_t least = (size_t)(row < 4096 ? 8 : 32) << 20;
+  const size_t piece = (size_t)(bytes < ((size_t)24 << 20) ? 128 : 256) << 10;
+  return bytes >= least && row <= piece ? piece : 0;
+}
 
 // The page-locked blocks of large copies, for all handles of the process: a
 // copy takes one and gives it back when it is done with it; up to two wait for
 // the next copies, until the last handle is destroyed.
 struct PieceBlocks {
+  struct Block {
+    void* p = nullptr;
+    size_t bytes = 0;
+  };
   std::mutex mutex;
-  void* idle[2] = {};
-  int nidle = 0, handles = 0;
+  Block idle[2];
+  int handles = 0;
   static PieceBlocks& get() {
     static PieceBlocks* p = new PieceBlocks;  // outlives every handle
     return *p;
   }
-  void* take() {
+  Block take(size_t bytes) {
     {
       std::lock_guard<std::mutex> lock(mutex);
-      if (nidle > 0) return idle[--nidle];
+      for (Block& b : idle)
+        if (b.bytes >= bytes) {
+          const Block t = b;
+          b = Block{};
+          return t;
+        }
     }
-    void* p = nullptr;
-    return cudaHostAlloc(&p, kPieceBlock, cudaHostAllocPortable) == cudaSuccess ? p : nullptr;
+    Block t;
+    if (cudaHostAlloc(&t.p, bytes, cudaHostAllocPortable) != cudaSuccess) return Block{};
+    t.bytes = bytes;
+    return t;
   }
-  void give(void* p) {
+  void give(Block t) {
     {
       std::lock_guard<std::mutex> lock(mutex);
-      if (handles > 0 && nidle < 2) {
-        idle[nidle++] = p;
-        return;
-      }
+      Block& least = idle[0].bytes <= idle[1].bytes ? idle[0] : idle[1];
+      if (handles > 0 && t.bytes > least.bytes) std::swap(t, least);
     }
-    cudaFreeHost(p);
+    if (t.p) cudaFreeHost(t.p);
   }
   void count(int d) {
-    void* drop[2] = {};
+    Block drop[2];
     {
       std::lock_guard<std::mutex> lock(mutex);
       handles += d;
-      if (handles == 0)
-        while (nidle > 0) {
-          --nidle;
-          drop[nidle] = idle[nidle];
-        }
+      if (handles == 0) std::swap(drop, idle);
     }
-    for (void* p : drop)
-      if (p) cudaFreeHost(p);
+    for (const Block& b : drop)
+      if (b.p) cudaFreeHost(b.p);
   }
 };
 
@@ -1640,20 +1655,20 @@ static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir, bool& t
   };
   const int64_t rows = 2 * task.rows;
   const size_t row_bytes = sizeof(double) * task.e0;
-  auto launch = [&](double* packed, int64_t r0, int64_t r1) {
+  auto launch = [&](cudaStream_t st, double* packed, int64_t r0, int64_t r1) {
     RowsTask t = task;
     t.packed = packed - r0 * task.e0;  // so that row r0 lies at `packed`
     const int64_t warps = (r1 - r0) * ((task.e0 + ROW_PART - 1) / ROW_PART);
     const unsigned g = (unsigned)std::max<int64_t>(1, std::min<int64_t>((warps + 7) / 8, 592));
-    if (dir == 0) k_rows<true><<<g, 256, 0, h->stream>>>(t, r0, r1);
-    else k_rows<false><<<g, 256, 0, h->stream>>>(t, r0, r1);
+    if (dir == 0) k_rows<true><<<g, 256, 0, st>>>(t, r0, r1);
+    else k_rows<false><<<g, 256, 0, st>>>(t, r0, r1);
     return cudaGetLastError();
   };
   if (row_bytes * rows <= kBounceBytes) {
     double* pin = static_cast<double*>(pin_reserve(h, row_bytes * rows));
     if (!pin) return none();
     if (dir == 0) std::memcpy(pin, host, row_bytes * rows);
-    CU(launch(pin, 0, rows));
+    CU(launch(h->stream, pin, 0, rows));
     ++h->stats.launches;
     if (dir == 0) {
       h->pin_busy = true;
@@ -1663,28 +1678,40 @@ static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir, bool& t
     }
     return BSAM_OK;
   }
-  const int64_t per = (int64_t)(kPieceBytes / row_bytes);
+  const size_t piece = piece_bytes(row_bytes * rows, row_bytes);
+  const int64_t per = (int64_t)(piece / row_bytes);
   const int64_t pieces = (rows + per - 1) / per;
   for (cudaEvent_t& e : h->slot_ev)
     if (!e) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
-  char* pin = static_cast<char*>(PieceBlocks::get().take());
-  if (!pin) return none();
+  for (cudaStream_t& st : h->copy_streams)
+    if (!st && cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking) != cudaSuccess)
+      return none();
+  const PieceBlocks::Block block = PieceBlocks::get().take(2 * kCopyThreads * piece);
+  if (!block.p) return none();
+  char* pin = static_cast<char*>(block.p);
   const int nt = (int)std::max(1u, std::min((unsigned)kCopyThreads,
                                             std::thread::hardware_concurrency()));
-  std::atomic<int> failed{(int)cudaSuccess};
+  // Thread 0 copies on the handle's stream, the others on their own, which take up
+  // where the handle's stands and are waited for before the call returns.
+  auto stream = [&](int t) { return t == 0 ? h->stream : h->copy_streams[t - 1]; };
+  std::atomic<int> failed{(int)cudaEventRecord(h->slot_ev[0], h->stream)};
+  for (int t = 1; t < nt; ++t)
+    if (failed.load() == (int)cudaSuccess)
+      failed.store((int)cudaStreamWaitEvent(stream(t), h->slot_ev[0], 0));
   // Thread t takes pieces t, t + nt, ..., the k-th of them in its slot k % 2.
   auto work = [&](int t) {
-    cudaError_t e = cudaSetDevice(h->device);
+    cudaError_t e = (cudaError_t)failed.load();
+    if (e == cudaSuccess) e = cudaSetDevice(h->device);
     auto first = [&](int64_t k) { return (t + k * nt) * per; };
     auto last = [&](int64_t k) { return std::min(rows, first(k) + per); };
     auto buf = [&](int64_t k) {
-      return reinterpret_cast<double*>(pin + (2 * t + (int)(k & 1)) * kPieceBytes);
+      return reinterpret_cast<double*>(pin + (2 * t + (int)(k & 1)) * piece);
     };
     auto ev = [&](int64_t k) { return h->slot_ev[2 * t + (int)(k & 1)]; };
     const int64_t n = (pieces - t + nt - 1) / nt;
     auto issue = [&](int64_t k) {
-      if (e == cudaSuccess) e = launch(buf(k), first(k), last(k));
-      if (e == cudaSuccess) e = cudaEventRecord(ev(k), h->stream);
+      if (e == cudaSuccess) e = launch(stream(t), buf(k), first(k), last(k));
+      if (e == cudaSuccess) e = cudaEventRecord(ev(k), stream(t));
     };
     if (dir != 0)
       for (int64_t k = 0; k < std::min<int64_t>(2, n); ++k) issue(k);
@@ -1703,6 +1730,8 @@ static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir, bool& t
         if (k + 2 < n) issue(k + 2);
       }
     }
+    const cudaError_t done = cudaStreamSynchronize(stream(t));
+    if (e == cudaSuccess) e = done;
     if (e != cudaSuccess) failed.store((int)e);
   };
   // The shares of threads that cannot be had are done by this one.
@@ -1716,9 +1745,7 @@ static int copy_state(bsam_gpu* h, RowsTask task, double* host, int dir, bool& t
   for (int t = started; t < nt; ++t) work(t);
   for (auto& t : pool) t.join();
   h->stats.launches += pieces;
-  const cudaError_t done = cudaStreamSynchronize(h->stream);  // the block's next user may write it
-  if (done != cudaSuccess) failed.store((int)done);
-  PieceBlocks::get().give(pin);
+  PieceBlocks::get().give(block);
   if (failed.load() != (int)cudaSuccess)
     return fail(h, BSAM_ERR_CUDA,
                 std::string("field copy: ") + cudaGetErrorString((cudaError_t)failed.load()));
@@ -1747,8 +1774,7 @@ static int copy_field(bsam_gpu* h, int patch, int field, double* host, int dir) 
       // With the ghost ring every row of every plane sits at stride sy on the
       // device (sz = sy * (n1 + 2)).
       const size_t bytes = 2 * hcomp * sizeof(double);
-      const bool pieces = bytes >= kThreadedBytes && e0 * sizeof(double) <= kPieceBytes;
-      if (bytes <= kBounceBytes || pieces) {
+      if (bytes <= kBounceBytes || piece_bytes(bytes, e0 * sizeof(double)) > 0) {
         double* dev1;
         const int rc1 = field_ptr(h, patch, field, 1, &dev1, &interior);
         if (rc1) return fail(h, rc1, "field not held for this patch");
@@ -2567,6 +2593,8 @@ int bsam_gpu_destroy(bsam_gpu* h) {
   if (h->h_pin) cudaFreeHost(h->h_pin);
   for (cudaEvent_t e : h->slot_ev)
     if (e) cudaEventDestroy(e);
+  for (cudaStream_t st : h->copy_streams)
+    if (st) cudaStreamDestroy(st);
   if (h->spare_arena) cudaFree(h->spare_arena);
   if (h->d_stash) cudaFree(h->d_stash);
   if (h->d_stash_spans) cudaFree(h->d_stash_spans);

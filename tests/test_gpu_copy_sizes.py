@@ -39,13 +39,18 @@ def test_fields_come_back_as_put(gpu_lib, mx):
         assert np.array_equal(out, b)
 
 
-@pytest.mark.parametrize("mx", [(510, 8), (512, 1100), (1030, 1024), (2046, 300), (5000, 220),
-                                (4094, 2)])
-def test_long_rows(gpu_lib, mx):
-    """Rows of several parts, a warp each, on every copy path."""
+# Rows of several parts (a warp each), and pieces of either size: rows below 4 KB
+# from 8 MiB (128 KB a piece, 256 from 24 MiB), longer rows from 32 MiB.
+@pytest.mark.parametrize("mx", [(510, 8), (4094, 2), (400, 1280), (400, 1310), (508, 1100),
+                                (30, 20000), (400, 4000), (1030, 1024), (2046, 1020),
+                                (2046, 1030), (5000, 424), (62, 62, 130), (40, 200, 190)])
+def test_long_rows_and_pieces(gpu_lib, mx):
+    nd = len(mx)
     rng = np.random.default_rng(sum(mx))
-    prob = W.Problem(ndims=2, mx=mx + (1,), eps=0.02, dt=1e-4, nsteps=1, qerrortol=1e-8,
-                     xupper=(1.0, mx[1] / mx[0], 1.0), c0=np.full(int(np.prod(mx)), 0.5))
+    h = 1.0 / mx[0]
+    prob = W.Problem(ndims=nd, mx=mx + (1,) * (3 - nd), eps=0.02, dt=1e-4, nsteps=1,
+                     qerrortol=1e-8, xupper=tuple([n * h for n in mx] + [1.0] * (3 - nd)),
+                     c0=np.full(int(np.prod(mx)), 0.5))
     a = np.asfortranarray(rng.standard_normal(tuple(m + 2 for m in mx) + (2,)))
     out = np.zeros_like(a, order="F")
     with B.Solver(prob) as s:
@@ -61,7 +66,7 @@ sys.path.insert(0, sys.argv[1])
 import bsam_b200 as B
 from bsam_b200 import workloads as W
 
-mx = (1022, 1024)
+mx = (400, 2600)
 prob = W.Problem(ndims=2, mx=mx + (1,), eps=0.02, dt=1e-4, nsteps=1, qerrortol=1e-8,
                  xupper=(1.0, mx[1] / mx[0], 1.0), c0=np.full(int(np.prod(mx)), 0.5))
 shape = tuple(m + 2 for m in mx) + (2,)
