@@ -19,7 +19,6 @@
 
 #include <algorithm>
 #include <mutex>
-#include <type_traits>
 
 #include "../../include/bsam_gpu.h"
 #include "bsam_types.h"
@@ -69,103 +68,169 @@ int scratch_for_device(int device, double** out) {
 // Lane l holds columns l and l + 32, which keeps every load whole lines; the tree's
 // pairs (columns 2m, 2m + 1) then meet across neighbouring lanes, its lanes m and
 // m + 16 within one.  Bound by HBM latency: a tile's four rows of two columns
-// unrolled keep their loads in flight, for which a thread needs 128 registers (4096^2,
-// 537 MB: 100 us = 5.3 TB/s with two CTAs per SM; 120 with three of 80
-// registers or four of 64.  128^3 18.6 against 25, 256^3 120 against 252.  Warps of
-// 32 columns with sums in an order of their own took 113, 23 and 167.)
+// unrolled keep their loads in flight, for which a thread needs 128 registers
+// (4096^2, 537 MB: 92 us = 5.8 TB/s; with pieces of 16 rows 100, and then with three
+// CTAs per SM of 80 registers or four of 64 120.  128^3 17.9, 256^3 128.  Warps of 32
+// columns with sums in an order of their own took 113, 23 and 167.)
 constexpr int NORM_WARPS = 8;
 constexpr int NORM_CTAS_PER_SM = 2;
-template <int D>
-__global__ void __launch_bounds__(32 * NORM_WARPS, NORM_CTAS_PER_SM)
-    k_resid_norm_noalloc(DevPatch P, const double* __restrict__ fbase, int64_t fsy,
-                         int64_t fsz, int64_t fcomp, int nseg, int nchunk, int rows,
-                         int64_t pieces, int tiles_y, double* __restrict__ scratch) {
-  next_may_launch();
+
+struct NormArgs {
+  const double *q0, *q1, *f;  // element (0, 0, 0) of q's components, (1, 1, 1) of f's first
+  int64_t sy, sz, fsy, fsz, fcomp;
+  double tmp1, tmp2, alpha;
+  int64_t pieces;
+  int n0, n1, nseg, nchunk, rows, tiles_y;
+};
+
+// Piece w: its tiles' sums go to out(tile, sum), by lane 0.
+template <int D, class Out>
+__device__ __forceinline__ void norm_piece(const NormArgs& P, int64_t w, Out&& out) {
   const int lane = threadIdx.x & 31;
   constexpr unsigned FULL = 0xffffffffu;
-  for (int64_t w = (int64_t)blockIdx.x * NORM_WARPS + (threadIdx.x >> 5); w < pieces;
-       w += (int64_t)gridDim.x * NORM_WARPS) {
-    const int64_t chunks = w / nseg;
-    const int seg = (int)(w - chunks * nseg);
-    const int plane = (int)(chunks / nchunk);
-    const int j0 = (int)(chunks - (int64_t)plane * nchunk) * rows + 1;
-    const int j1 = min(j0 + rows - 1, P.n[1]);
-    const int k = D == 3 ? plane + 1 : 0;
-    const int i = seg * TILE_X + lane + 1;
-    const bool on[2] = {i <= P.n[0], i + 32 <= P.n[0]};
-    const double* q0 = static_cast<const double*>(P.q[0]) + cidx(P, i, j0, k);
-    const double* q1 = static_cast<const double*>(P.q[1]) + cidx(P, i, j0, k);
-    const double* f = fbase + (int64_t)(i - 1) + (int64_t)(j0 - 1) * fsy +
-                      (int64_t)(D == 3 ? plane : 0) * fsz;
-    // Lanes beyond the row load nothing and add nothing.
-    auto ld = [&](const double* p, int h) { return on[h] ? p[32 * h] : 0.0; };
-    double ps[2], pc[2], ms[2], mc[2];
+  const int64_t chunks = w / P.nseg;
+  const int seg = (int)(w - chunks * P.nseg);
+  const int plane = (int)(chunks / P.nchunk);
+  const int j0 = (int)(chunks - (int64_t)plane * P.nchunk) * P.rows + 1;
+  const int j1 = min(j0 + P.rows - 1, P.n1);
+  const int k = D == 3 ? plane + 1 : 0;
+  const int i = seg * TILE_X + lane + 1;
+  const bool on[2] = {i <= P.n0, i + 32 <= P.n0};
+  const int64_t c = i + j0 * P.sy + (D == 3 ? k * P.sz : 0);
+  const double *q0 = P.q0 + c, *q1 = P.q1 + c;
+  const double* f = P.f + (i - 1) + (j0 - 1) * P.fsy + (D == 3 ? plane * P.fsz : 0);
+  // Lanes beyond the row load nothing and add nothing.
+  auto ld = [&](const double* p, int h) { return on[h] ? p[32 * h] : 0.0; };
+  double ps[2], pc[2], ms[2], mc[2];
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    ps[h] = ld(q0 - P.sy, h);
+    pc[h] = ld(q0, h);
+    ms[h] = ld(q1 - P.sy, h);
+    mc[h] = ld(q1, h);
+  }
+  int64_t tile = ((int64_t)plane * P.tiles_y + (j0 - 1) / TILE_Y) * P.nseg + seg;
+  // The squares of row r of the current tile; the pointers move on.
+  auto row = [&](double (&v)[2]) {
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-      ps[h] = ld(q0 - P.sy, h);
-      pc[h] = ld(q0, h);
-      ms[h] = ld(q1 - P.sy, h);
-      mc[h] = ld(q1, h);
+      Problem::Stencil<double, D> s;
+      s.pc = pc[h];
+      s.mc = mc[h];
+      s.pm[0] = ld(q0 - 1, h);
+      s.pp[0] = ld(q0 + 1, h);
+      s.mm[0] = ld(q1 - 1, h);
+      s.mp[0] = ld(q1 + 1, h);
+      s.pm[1] = ps[h];
+      s.pp[1] = ld(q0 + P.sy, h);
+      s.mm[1] = ms[h];
+      s.mp[1] = ld(q1 + P.sy, h);
+      if (D == 3) {
+        s.pm[D - 1] = ld(q0 - P.sz, h);
+        s.pp[D - 1] = ld(q0 + P.sz, h);
+        s.mm[D - 1] = ld(q1 - P.sz, h);
+        s.mp[D - 1] = ld(q1 + P.sz, h);
+      }
+      double o0, o1;
+      Problem::OperatorCell<double, D>(s, P.tmp1, P.tmp2, P.alpha, o0, o1);
+      const double r0 = ld(f, h) - o0, r1 = ld(f + P.fcomp, h) - o1;
+      v[h] = on[h] ? r0 * r0 + r1 * r1 : 0.0;
+      ps[h] = pc[h];
+      ms[h] = mc[h];
+      pc[h] = s.pp[1];
+      mc[h] = s.mp[1];
     }
-    int64_t tile = ((int64_t)plane * tiles_y + (j0 - 1) / TILE_Y) * nseg + seg;
-    // The squares of row r of the current tile; the pointers move on.
-    auto row = [&](double (&v)[2]) {
+    q0 += P.sy;
+    q1 += P.sy;
+    f += P.fsy;
+  };
+  for (int jt = j0; jt <= j1; jt += TILE_Y, tile += P.nseg) {
+    double v[TILE_Y][2] = {};
+    if (jt + TILE_Y - 1 <= j1) {  // without conditions between the rows' loads
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        Problem::Stencil<double, D> s;
-        s.pc = pc[h];
-        s.mc = mc[h];
-        s.pm[0] = ld(q0 - 1, h);
-        s.pp[0] = ld(q0 + 1, h);
-        s.mm[0] = ld(q1 - 1, h);
-        s.mp[0] = ld(q1 + 1, h);
-        s.pm[1] = ps[h];
-        s.pp[1] = ld(q0 + P.sy, h);
-        s.mm[1] = ms[h];
-        s.mp[1] = ld(q1 + P.sy, h);
-        if (D == 3) {
-          s.pm[D - 1] = ld(q0 - P.sz, h);
-          s.pp[D - 1] = ld(q0 + P.sz, h);
-          s.mm[D - 1] = ld(q1 - P.sz, h);
-          s.mp[D - 1] = ld(q1 + P.sz, h);
-        }
-        double o0, o1;
-        Problem::OperatorCell<double, D>(s, P.tmp1, P.tmp2, P.alpha, o0, o1);
-        const double r0 = ld(f, h) - o0, r1 = ld(f + fcomp, h) - o1;
-        v[h] = on[h] ? r0 * r0 + r1 * r1 : 0.0;
-        ps[h] = pc[h];
-        ms[h] = mc[h];
-        pc[h] = s.pp[1];
-        mc[h] = s.mp[1];
-      }
-      q0 += P.sy;
-      q1 += P.sy;
-      f += fsy;
-    };
-    for (int jt = j0; jt <= j1; jt += TILE_Y, tile += nseg) {
-      double v[TILE_Y][2] = {};
-      if (jt + TILE_Y - 1 <= j1) {  // without conditions between the rows' loads
+      for (int r = 0; r < TILE_Y; ++r) row(v[r]);
+    } else {
 #pragma unroll
-        for (int r = 0; r < TILE_Y; ++r) row(v[r]);
-      } else {
-#pragma unroll
-        for (int r = 0; r < TILE_Y - 1; ++r)
-          if (jt + r <= j1) row(v[r]);
-      }
-      double sum = 0.0;
-#pragma unroll
-      for (int r = 0; r < TILE_Y; ++r) {
-        // Lane 2m: the sums of pairs m and m + 16, then the tree's further levels.
-        const double a = v[r][0] + __shfl_xor_sync(FULL, v[r][0], 1);
-        const double b = v[r][1] + __shfl_xor_sync(FULL, v[r][1], 1);
-        double s = a + b;
-#pragma unroll
-        for (int o = 16; o > 1; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
-        sum += s;
-      }
-      if (lane == 0) scratch[tile] = sum;
+      for (int r = 0; r < TILE_Y - 1; ++r)
+        if (jt + r <= j1) row(v[r]);
     }
+    double sum = 0.0;
+#pragma unroll
+    for (int r = 0; r < TILE_Y; ++r) {
+      // Lane 2m: the sums of pairs m and m + 16, then the tree's further levels.
+      const double a = v[r][0] + __shfl_xor_sync(FULL, v[r][0], 1);
+      const double b = v[r][1] + __shfl_xor_sync(FULL, v[r][1], 1);
+      double s = a + b;
+#pragma unroll
+      for (int o = 16; o > 1; o >>= 1) s += __shfl_xor_sync(FULL, s, o);
+      sum += s;
+    }
+    if (lane == 0) out(tile, sum);
   }
+}
+
+template <int D>
+__global__ void __launch_bounds__(32 * NORM_WARPS, NORM_CTAS_PER_SM)
+    k_resid_norm_noalloc(const NormArgs P, double* __restrict__ scratch) {
+  next_may_launch();
+  for (int64_t w = (int64_t)blockIdx.x * NORM_WARPS + (threadIdx.x >> 5); w < P.pieces;
+       w += (int64_t)gridDim.x * NORM_WARPS)
+    norm_piece<D>(P, w, [&](int64_t tile, double sum) { scratch[tile] = sum; });
+}
+
+__device__ __forceinline__ void cluster_arrive() {
+  asm volatile("barrier.cluster.arrive.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+}
+// Stores into the cluster's first CTA, at the place of this CTA's own `p`.
+__device__ __forceinline__ void store_first(double* p, double v) {
+  uint32_t at;
+  asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(p)));
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(v) : "memory");
+}
+
+// block_sum of BLOCK_THREADS threads by the first of a larger CTA, then the norm.
+__device__ __forceinline__ void norm_out(double x, double denom, double* out) {
+  __shared__ double red[BLOCK_THREADS / 32];
+  if (threadIdx.x < BLOCK_THREADS) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = x;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double total = 0.0;
+    for (int w = 0; w < BLOCK_THREADS / 32; ++w) total += red[w];
+    out[0] = sqrt(total / denom);
+    out[1] = total;
+  }
+}
+
+// Patches of at most a tile per warp by one cluster in one launch, the tiles' sums in
+// its first CTA's shared memory: such a call is bound by the host, where a second
+// launch costs 2 us (101 x 200 from Python 9.7 us a call against 11.6; 309 x 105, 135
+// tiles, takes 8.3 us on the device this way and 6.8 by two launches).
+constexpr int SMALL_CTAS = 8, SMALL_THREADS = 512, SMALL_WARPS = SMALL_CTAS * SMALL_THREADS / 32;
+constexpr int SMALL_TILES = 128;
+template <int D>
+__global__ void __cluster_dims__(SMALL_CTAS, 1, 1) __launch_bounds__(SMALL_THREADS, 1)
+    k_norm_small(const NormArgs P, int tiles, double denom, double* __restrict__ out) {
+  __shared__ double part[SMALL_TILES];
+  cluster_arrive();
+  cluster_wait();  // every CTA of the cluster runs: its memory may be written
+  for (int64_t w = (int64_t)blockIdx.x * (SMALL_THREADS / 32) + (threadIdx.x >> 5); w < P.pieces;
+       w += SMALL_WARPS)
+    norm_piece<D>(P, w, [&](int64_t tile, double sum) { store_first(part + tile, sum); });
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  if (blockIdx.x != 0) return;
+  double s = 0.0;
+  if (threadIdx.x < BLOCK_THREADS)
+    for (int b = threadIdx.x; b < tiles; b += BLOCK_THREADS) s += part[b];
+  norm_out(s, denom, out);
 }
 
 // The sum of the tiles' sums in the solver's order (last_block_sum, kernels.cuh:
@@ -205,6 +270,7 @@ __global__ void __cluster_dims__(TOTAL_CTAS, 1, 1) __launch_bounds__(TOTAL_THREA
   __shared__ double sums[BLOCK_THREADS];
   const int lane = threadIdx.x % TOTAL_SUMS, row = threadIdx.x / TOTAL_SUMS;
   const int first = blockIdx.x * TOTAL_SUMS + lane;
+  cluster_arrive();
   after_previous();
   double v[TOTAL_LOADS];
 #pragma unroll
@@ -226,35 +292,22 @@ __global__ void __cluster_dims__(TOTAL_CTAS, 1, 1) __launch_bounds__(TOTAL_THREA
 #pragma unroll 16
       for (int r = 0; r < n; ++r) s += part[r][lane];
   }
-  if (row == 0) {
-    const uint32_t a = (uint32_t)__cvta_generic_to_shared(&sums[first]);
-    uint32_t at;
-    asm("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(at) : "r"(a));
-    asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(at), "d"(s) : "memory");
-  }
-  asm volatile("barrier.cluster.arrive.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
-  if (blockIdx.x != 0) return;
-  // block_sum of BLOCK_THREADS threads.
-  __shared__ double red[BLOCK_THREADS / 32];
-  if (threadIdx.x < BLOCK_THREADS) {
-    double x = sums[threadIdx.x];
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = x;
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double total = 0.0;
-    for (int w = 0; w < BLOCK_THREADS / 32; ++w) total += red[w];
-    out[0] = sqrt(total / denom);
-    out[1] = total;
-  }
+  cluster_wait();  // every CTA of the cluster runs: its memory may be written
+  if (row == 0) store_first(sums + first, s);
+  __syncwarp();
+  cluster_arrive();
+  cluster_wait();
+  if (blockIdx.x == 0) norm_out(threadIdx.x < BLOCK_THREADS ? sums[threadIdx.x] : 0.0, denom, out);
 }
 
-template <int D, class... A>
-cudaError_t launch_norm(unsigned ctas, int tiles, cudaStream_t s, double* scratch, double denom, double* out,
-                        A... args) {
-  k_resid_norm_noalloc<D><<<ctas, 32 * NORM_WARPS, 0, s>>>(args..., scratch);
+template <int D>
+cudaError_t launch_norm(const NormArgs& P, unsigned ctas, int tiles, cudaStream_t s,
+                        double* scratch, double denom, double* out) {
+  if (tiles <= SMALL_TILES) {
+    k_norm_small<D><<<SMALL_CTAS, SMALL_THREADS, 0, s>>>(P, tiles, denom, out);
+    return cudaGetLastError();
+  }
+  k_resid_norm_noalloc<D><<<ctas, 32 * NORM_WARPS, 0, s>>>(P, scratch);
   const cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg{};
@@ -267,7 +320,8 @@ cudaError_t launch_norm(unsigned ctas, int tiles, cudaStream_t s, double* scratc
   at.val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  (void)cudaLaunchKernelEx(&cfg, few ? k_norm_total_few : k_norm_total, (const double*)scratch, tiles, denom, out);
+  (void)cudaLaunchKernelEx(&cfg, few ? k_norm_total_few : k_norm_total, (const double*)scratch,
+                           tiles, denom, out);
   return cudaGetLastError();
 }
 
@@ -290,52 +344,57 @@ extern "C" int bsam_gpu_resid_norm_noalloc(int device, int ndims, const int32_t*
 
   int prev = -1;
   if (cudaGetDevice(&prev) != cudaSuccess) return BSAM_ERR_NODEVICE;
-  if (cudaSetDevice(device) != cudaSuccess) return BSAM_ERR_NODEVICE;
+  if (prev != device && cudaSetDevice(device) != cudaSuccess) return BSAM_ERR_NODEVICE;
   double* scratch = nullptr;
   int rc = scratch_for_device(device, &scratch);
   if (rc == BSAM_OK) {
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    DevPatch P{};
-    P.ndims = ndims;
-    for (int d = 0; d < 3; ++d) P.n[d] = (int32_t)n[d];
+    NormArgs P{};
+    P.n0 = (int)n[0];
+    P.n1 = (int)n[1];
     P.sy = n[0] + 2;
     P.sz = ndims == 3 ? (n[0] + 2) * (n[1] + 2) : 0;
     const int64_t qcomp = (n[0] + 2) * (n[1] + 2) * (ndims == 3 ? n[2] + 2 : 1);
-    P.q[0] = const_cast<double*>(q);
-    P.q[1] = const_cast<double*>(q) + qcomp;
+    P.q0 = q;
+    P.q1 = q + qcomp;
+    P.f = f;
+    P.fsy = n[0];
+    P.fsz = n[0] * n[1];
+    P.fcomp = n[0] * n[1] * n[2];
     // Operator constants computed as in problem.f90:246-248.
     const double h2 = dx * dx;
-    P.h = dx;
     P.alpha = alpha;
     P.tmp1 = dt / h2;
     P.tmp2 = eps * eps / h2;
     const double denom = (double)(2 * n[0] * n[1] * n[2]);
-    const int64_t fsy = n[0], fsz = n[0] * n[1], fcomp = n[0] * n[1] * n[2];
-    const int64_t nseg = tiles_x;
-    // Rows per piece, whole tiles: those for which the warps, each at its share of
-    // the pieces, take the fewest rows (the row above a piece is loaded again).
-    const int64_t kCtas = B200_SMS * NORM_CTAS_PER_SM;
-    int64_t rows = TILE_Y, least = INT64_MAX;
-    for (int64_t r = TILE_Y; r <= 32 * TILE_Y; r += TILE_Y) {
-      const int64_t all = nseg * ((n[1] + r - 1) / r) * n[2];
-      const int64_t cost = (all + kCtas * NORM_WARPS - 1) / (kCtas * NORM_WARPS) * (r + 1);
-      if (cost < least) {
-        least = cost;
-        rows = r;
-      }
+    P.nseg = (int)tiles_x;
+    P.tiles_y = (int)tiles_y;
+    // Rows per piece, whole tiles: as many as let the warps finish in one to four
+    // pieces each, whichever takes the fewest rows (the row above a piece is loaded
+    // again), at most 128.  (In 32-bit arithmetic and few steps: trying every size took
+    // the host a microsecond.)
+    constexpr int kCtas = B200_SMS * NORM_CTAS_PER_SM;
+    const int warps = tiles <= SMALL_TILES ? SMALL_WARPS : kCtas * NORM_WARPS;
+    const int columns = (int)(tiles_x * n[2]);
+    int least = 0;
+    for (int turns = 1; turns <= 4; ++turns) {
+      const int chunks = std::max(1, turns * warps / columns);
+      const int r = std::min(32, ((int)tiles_y + chunks - 1) / chunks) * TILE_Y;
+      const int at = ((int)n[1] + r - 1) / r * columns;
+      const int cost = (at + warps - 1) / warps * (r + 1);
+      if (turns > 1 && cost >= least) continue;
+      least = cost;
+      P.rows = r;
+      P.pieces = at;
     }
-    const int64_t nchunk = (n[1] + rows - 1) / rows;
-    const int64_t pieces = nseg * nchunk * n[2];
-    const int64_t ctas = std::min<int64_t>(kCtas, (pieces + NORM_WARPS - 1) / NORM_WARPS);
-    auto launch = [&](auto dim) {
-      return launch_norm<decltype(dim)::value>((unsigned)ctas, (int)tiles, s, scratch, denom, out, P, f, fsy,
-                                               fsz, fcomp, (int)nseg, (int)nchunk, (int)rows,
-                                               pieces, (int)tiles_y);
-    };
-    const cudaError_t e = ndims == 2 ? launch(std::integral_constant<int, 2>{})
-                                     : launch(std::integral_constant<int, 3>{});
+    P.nchunk = (int)(P.pieces / columns);
+    const unsigned ctas =
+        (unsigned)std::min<int64_t>(kCtas, (P.pieces + NORM_WARPS - 1) / NORM_WARPS);
+    const cudaError_t e =
+        ndims == 2 ? launch_norm<2>(P, ctas, (int)tiles, s, scratch, denom, out)
+                   : launch_norm<3>(P, ctas, (int)tiles, s, scratch, denom, out);
     if (e != cudaSuccess) rc = BSAM_ERR_CUDA;
   }
-  cudaSetDevice(prev);
+  if (prev != device) cudaSetDevice(prev);
   return rc;
 }

@@ -105,6 +105,7 @@ def test_captured_call_replays(gpu_lib):
 
 
 @pytest.mark.parametrize("mx", [(2, 2), (66, 6), (130, 34), (200, 72), (62, 1030), (512, 512),
+                                (64, 512), (64, 514), (2048, 256), (2048, 258),
                                 (2048, 1030), (6, 10, 4), (70, 10, 6), (128, 66, 34),
                                 (200, 96, 64)])
 def test_norm_is_the_solvers_bit_for_bit(gpu_lib, mx):
