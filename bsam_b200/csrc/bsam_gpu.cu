@@ -1197,8 +1197,11 @@ static int set_hierarchy(bsam_gpu* h, int npatch, const bsam_patch_desc* patches
     const bool fuse3 = h->tuning.fuse_smoother != 0 && nd == 3 && finestlevel == 0 && !periodic &&
                        !(P.delta && P.prec == PREC_F64) && P.n[0] >= fmin && P.n[1] >= fmin &&
                        P.n[2] >= fmin;
+    // (Levels with more rows of tiles than a grid holds, above 1048560 rows of cells,
+    // run a launch per pass.)
     const bool fuse2 = stages2 && nd == 2 && h->tuning.bottom_cells >= 0 && d.level <= 0 &&
-                       h->rp.nsmoothingpasses <= 2 && alone[d.level - minlevel];
+                       h->rp.nsmoothingpasses <= 2 && alone[d.level - minlevel] &&
+                       P.n[1] <= 16 * MAX_GRID_Y;
     P.fused = (fuse3 || fuse2) && in_vcycle && d.parent >= 0 && d.level > h->bottom_level ? 1 : 0;
     if (P.fused && nd == 3) {
       const int ftx = P.prec == PREC_F32 ? Fused3<float>::TX : Fused3<double>::TX;

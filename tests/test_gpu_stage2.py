@@ -63,6 +63,14 @@ def test_wide_levels(gpu_lib, mx, faces, precision):
     same(solve(prob, precision, 0), solve(prob, precision, -1))
 
 
+# 65535 tiles of 16 rows are a grid's most: longer columns run a launch per pass.
+@pytest.mark.parametrize("precision", [B.PREC_FP64, B.PREC_MIXED])
+@pytest.mark.parametrize("mx", [(2, 16 * 65535), (2, 16 * 65535 + 2), (4, 2 ** 21)])
+def test_columns_longer_than_a_grid(gpu_lib, mx, precision):
+    prob = problem(mx, "neumann")
+    same(solve(prob, precision, 0), solve(prob, precision, -1))
+
+
 @pytest.mark.parametrize("faces", ["user", "periodic"])
 def test_first_sweep_reads_the_ghosts_as_given(gpu_lib, faces):
     prob = problem((64, 48), faces)
