@@ -80,8 +80,9 @@ int bsam_gpu_create(bsam_gpu** h, int device, const bsam_run_params* p);
  *                  level allows it: 3D levels.  2D levels at and below the
  *                  root, of one patch and at most two sweeps, always run as
  *                  such stages above the bottom chain, unless bottom_cells
- *                  is -1 or the second state that a stage needs (two more
- *                  fields a level, 268 MB at 4096^2 FP64) does not fit
+ *                  is -1, the second state that a stage needs (two more
+ *                  fields a level, 268 MB at 4096^2 FP64) does not fit, or
+ *                  the level has more than 1048560 rows
  *   fuse_min_n     smallest extent per dimension of a fused level
  *   chunk          planes (3D) / rows (2D) per streaming chunk, 0 = automatic
  *   bottom_cells   levels of at most this many cells run their whole part of
